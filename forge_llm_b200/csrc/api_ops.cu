@@ -252,9 +252,11 @@ int32_t forge_attention_flash(float* out, const float* q, const uint16_t* k_cach
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     int splits = attn_decode_splits((seq_len + FORGE_KV_PAGE - 1) / FORGE_KV_PAGE, num_kv_heads, 148, head_dim, num_heads / num_kv_heads);
     AsyncBuf ws(st), cnt(st);
-    FORGE_CUDA(ws.alloc(sizeof(float) * attn_decode_ws_floats(1, num_heads, head_dim, splits)));
-    FORGE_CUDA(cnt.alloc(sizeof(int) * num_kv_heads));
-    FORGE_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(int) * num_kv_heads, st));
+    if (const size_t fl = attn_decode_ws_floats(1, num_heads, head_dim, splits)) {
+        FORGE_CUDA(ws.alloc(sizeof(float) * fl));
+        FORGE_CUDA(cnt.alloc(sizeof(int) * num_kv_heads));
+        FORGE_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(int) * num_kv_heads, st));
+    }
     AttnDecodeArgs a{out, q, reinterpret_cast<const __half*>(k_cache), reinterpret_cast<const __half*>(v_cache), nullptr, 0, nullptr,
                      seq_len, 1, num_heads, num_kv_heads, head_dim, seq_len, static_cast<float*>(ws.p), static_cast<int*>(cnt.p), splits};
     return attn_decode(a, st);
@@ -300,9 +302,11 @@ int32_t forge_attention_sliding(float* out, const float* q, const uint16_t* k_ca
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     int splits = attn_decode_splits((seq_len + FORGE_KV_PAGE - 1) / FORGE_KV_PAGE, num_kv_heads, 148, head_dim, num_heads / num_kv_heads);
     AsyncBuf ws(st), cnt(st);
-    FORGE_CUDA(ws.alloc(sizeof(float) * attn_decode_ws_floats(1, num_heads, head_dim, splits)));
-    FORGE_CUDA(cnt.alloc(sizeof(int) * num_kv_heads));
-    FORGE_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(int) * num_kv_heads, st));
+    if (const size_t fl = attn_decode_ws_floats(1, num_heads, head_dim, splits)) {
+        FORGE_CUDA(ws.alloc(sizeof(float) * fl));
+        FORGE_CUDA(cnt.alloc(sizeof(int) * num_kv_heads));
+        FORGE_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(int) * num_kv_heads, st));
+    }
     AttnDecodeArgs a{out, q, reinterpret_cast<const __half*>(k_cache), reinterpret_cast<const __half*>(v_cache), nullptr, 0, nullptr,
                      seq_len, 1, num_heads, num_kv_heads, head_dim, seq_len, static_cast<float*>(ws.p), static_cast<int*>(cnt.p), splits, window};
     return attn_decode(a, st);

@@ -1,46 +1,50 @@
 // Single-query decode attention over the paged fp16 KV cache (replaces attention_flash,
 // crates/forgellm-codegen-cpu/src/emit.rs:657-715; GQA mapping kv_head = h / (nq/nkv), :660-666).
-// HBM-bound on K/V: the context is split over CTAs (split-KV); a producer lane pulls the CTA's pages - 64 rows of one
-// KV head, K and V - into a ring of shared-memory stages with 3-D tiled TMA copies (cp.async.bulk.tensor, mbarrier
-// completion; the tensor map spans this GPU's own pool), so the bytes in flight do not depend on registers or on
-// the instruction stream, and it starts before the dependency wait: every cached row but the newest was written by
-// earlier steps.  Four consumer warps read the rows from shared memory with 128-bit loads, every row shared by the
-// query heads of its group; the online-softmax state (m, l, acc) is f32.  Split partials are merged by the last CTA
-// to finish a KV head (atomic ticket), so no second launch is needed.  Every wait is bounded.
+//
+// What bounds it: for one sequence the chain launch -> query -> page -> merge, for many sequences the bytes of K and V.  The context is split
+// over CTAs; a producer lane pulls the CTA's pages - 64 rows of one KV head, K and V - into a ring of shared-memory stages with 3-D tiled TMA copies
+// (SWIZZLE_128B, boxes of 64 dimensions; the tensor map spans this GPU's own pool), before the dependency wait: every cached row but the
+// newest was written by earlier steps.
+//
+// Four consumer warps take sixteen keys of a page each, as mma.sync products: up to eight query heads of the group are rows 0..7 of the A tile as fp16 hi
+// parts and rows 8..15 as lo parts, so that one product serves both halves of the 22-bit query and a thread adds them from its own registers; the probabilities
+// enter their product with the values the same way.  Softmax state is f32.  A page costs a warp about forty tensor instructions at
+// head_dim 64 whatever the group; with scores and sums formed by fused multiply-adds (four heads per pass over the page) one page took 1.7 us.
+// The splits of a (sequence, KV head) are a cluster and merge through distributed shared memory; beyond eight splits (contexts past 128 pages) the
+// last CTA to finish merges partials from global memory (atomic ticket).  Every wait is bounded.
 #include <cuda.h>
 
 #include <algorithm>
 #include <mutex>
 
 #include "common.cuh"
+#include "mma.cuh"
+#include "tc5.cuh"
 
 namespace forge {
 
 namespace {
 
+using tc5::cluster_addr;
+using tc5::cluster_sync;
+
 constexpr int kThreads = 128;     // consumer threads (four warps); warp 4 is the producer
 constexpr int kBlock = kThreads + 32;
-constexpr int kStages = 4;        // most pages (K and V) in flight per CTA (a CTA with one or two pages takes a ring of two)
-constexpr int kMaxGroup = 16;  // query heads per KV head
-constexpr int kMaxSplits = 32;    // context splits per KV head (the merge keeps one partial per split in registers)
+constexpr int kStages = 4;        // most pages (K and V) in flight per CTA
+constexpr int kMaxGroup = 16;     // query heads per KV head
+constexpr int kHeads = 8;         // of them in one pass over the keys
+constexpr int kMaxSplits = 32;    // context splits per KV head
+constexpr int kClusterSplits = 8; // of them in a cluster
 constexpr uint32_t kSpin = 1u << 22;
-
-template <int HD> struct Seg { static constexpr int W = (HD == 64) ? 8 : 16, ACTIVE = HD / 8, RPW = 32 / W; };
+constexpr float kLog2e = 1.4426950408889634f;
 
 struct DecParams {
     AttnDecodeArgs a;
-    float scale;
+    float scale;  // of the scores, times log2 e
     int stages;   // ring depth of this launch (<= kStages)
 };
 
-__device__ __forceinline__ void unpack8(const uint4& v, float* f) {
-    const __half2* h = reinterpret_cast<const __half2*>(&v);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) { float2 t = __half22float2(h[i]); f[2 * i] = t.x; f[2 * i + 1] = t.y; }
-}
-
-// exp(x - m) with exp(-inf) = 0 and no NaN when both are -inf
-__device__ __forceinline__ float exp_rel(float x, float m) { return (x == -INFINITY) ? 0.f : __expf(x - m); }
+__device__ __forceinline__ float exp2_rel(float x, float m) { return x == -INFINITY ? 0.f : exp2f(x - m); }   // 0 for an empty part, never NaN
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
@@ -62,10 +66,10 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     }
     return false;
 }
-// one page of one KV head: box {head_dim, 1, 64 rows} at {0, kv head, row}
-__device__ __forceinline__ void tma_page(void* dst, const CUtensorMap* map, int kvh, int row, uint64_t* bar) {
+// 64 dimensions of one page of one KV head: box {64, 1, 64 rows} at {dimension, kv head, row}
+__device__ __forceinline__ void tma_page(void* dst, const CUtensorMap* map, int dim, int kvh, int row, uint64_t* bar) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-                 ::"r"(smem_u32(dst)), "l"(map), "r"(0), "r"(kvh), "r"(row), "r"(smem_u32(bar)) : "memory");
+                 ::"r"(smem_u32(dst)), "l"(map), "r"(dim), "r"(kvh), "r"(row), "r"(smem_u32(bar)) : "memory");
 }
 // the result in the form the caller asked for: f32, or fp16 hi (+ lo)
 __device__ __forceinline__ void store_out(const AttnDecodeArgs& a, size_t i, float x) {
@@ -91,27 +95,42 @@ __device__ __forceinline__ void store_out2(const AttnDecodeArgs& a, size_t i, fl
 }
 __device__ __forceinline__ void csync() { asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory"); }
 
-// SW: sliding-window instantiation (the full-attention one carries no window tests)
-// GC: query heads folded per pass over the keys: min(4, query heads per KV head), so that multi-head attention (one
-// query head per KV head) forms one score per key, not four
-template <int HD, bool SW, int GC>
-__global__ void __launch_bounds__(kBlock, (HD == 128 || GC == 4) ? 2 : 3) attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
-                                                             DecParams p) {
-    constexpr int W = Seg<HD>::W, ACTIVE = Seg<HD>::ACTIVE, RPW = Seg<HD>::RPW;
-    constexpr int PARTS = (kThreads / 32) * RPW;
-    constexpr int PAGE_BYTES = FORGE_KV_PAGE * HD * 2;
-    extern __shared__ __align__(1024) unsigned char ring[];   // [kStages][K page | V page]
+__device__ __forceinline__ void mma16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// two values as packed fp16 hi parts and lo parts
+__device__ __forceinline__ void split_h2(float x, float y, uint32_t& hi, uint32_t& lo) {
+    const __half2 h = __floats2half2_rn(x, y);
+    const float2 f = __half22float2(h);
+    const __half2 l = __floats2half2_rn(x - f.x, y - f.y);
+    hi = *reinterpret_cast<const uint32_t*>(&h);
+    lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+__device__ __forceinline__ float remote_f32(uint32_t addr) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+    return v;
+}
+
+// SW: sliding-window instantiation (the full-attention one carries no window tests); CL: the splits are a cluster
+template <int HD, bool SW, bool CL>
+__global__ void __launch_bounds__(kBlock, HD == 64 ? 3 : 2) attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, DecParams p) {
+    constexpr int BOXES = (HD + 63) / 64;                 // boxes of 64 dimensions (the second one of 96-wide heads is half zeros)
+    constexpr int BOX_BYTES = FORGE_KV_PAGE * 128;
+    constexpr int PAGE_BYTES = BOXES * BOX_BYTES;
+    constexpr int KS = HD / 16, NV = HD / 8;
+    extern __shared__ __align__(1024) unsigned char ring_raw[];   // [stages][K page | V page], then [warp][head][HD] sums
+    unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(ring_raw) + 1023) & ~uintptr_t(1023));
+    float* s_acc = reinterpret_cast<float*>(ring + size_t(p.stages) * 2 * PAGE_BYTES);   // in the end [head][HD] of the CTA
     __shared__ uint64_t full_bar[kStages], empty_bar[kStages];
-    __shared__ float s_m[PARTS][GC], s_l[PARTS][GC], s_w[PARTS][GC];
-    __shared__ float s_acc[PARTS][GC][HD];
-    __shared__ float s_fw[kMaxSplits][kMaxGroup];  // final merge: weight of split s for query head g
+    __shared__ float s_ml[4][kHeads][2], s_cml[kHeads][2];
+    __shared__ float s_fw[kMaxSplits][kMaxGroup];         // global merge: weight of split s for query head g
     __shared__ int s_last;
     const AttnDecodeArgs& a = p.a;
     pdl_trigger();
     const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int seg = lane / W, sl = lane % W;
-    const bool act = sl < ACTIVE;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lr = lane >> 2, lc = (lane & 3) * 2;
     const int G = a.nq / a.nkv, kvd = a.nkv * HD;
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], kThreads / 32); }
@@ -126,16 +145,12 @@ __global__ void __launch_bounds__(kBlock, (HD == 128 || GC == 4) ? 2 : 3) attn_d
     const int n_pages = (n_ctx + FORGE_KV_PAGE - 1) / FORGE_KV_PAGE;
     const int t_first = (SW && n_ctx > a.window) ? n_ctx - a.window : 0;  // sliding window: first position seen
     const size_t seq_base = a.page_table ? 0 : size_t(b) * a.max_ctx;  // contiguous: [batch][max_ctx][kvd]
-    const int part = warp * RPW + seg;
-    // positions per segment folded into the running softmax state in one step (a whole page per warp step when one
-    // query head leaves the registers for it)
-    constexpr int UNR = (GC == 1 && W == 16) ? 8 : 4;
 
     if (warp == kThreads / 32) {
         // ---- producer: the CTA's pages, once per pass over the query heads, as ring space frees up
         if (lane == 0) {
             int i = 0;
-            for (int g0 = 0; g0 < G; g0 += GC)
+            for (int g0 = 0; g0 < G; g0 += kHeads)
                 for (int lp = split; lp < n_pages; lp += a.splits) {
                     if (SW && (lp + 1) * FORGE_KV_PAGE <= t_first) continue;
                     const int st = i % p.stages, use = i / p.stages;
@@ -143,8 +158,11 @@ __global__ void __launch_bounds__(kBlock, (HD == 128 || GC == 4) ? 2 : 3) attn_d
                     const int row = a.row_base + int(seq_base) + (pt ? pt[lp] : lp) * FORGE_KV_PAGE;
                     unsigned char* dst = ring + size_t(st) * 2 * PAGE_BYTES;
                     mbar_expect_tx(&full_bar[st], 2 * PAGE_BYTES);
-                    tma_page(dst, &map_k, kvh, row, &full_bar[st]);
-                    tma_page(dst + PAGE_BYTES, &map_v, kvh, row, &full_bar[st]);
+#pragma unroll
+                    for (int x = 0; x < BOXES; ++x) {
+                        tma_page(dst + x * BOX_BYTES, &map_k, x * 64, kvh, row, &full_bar[st]);
+                        tma_page(dst + PAGE_BYTES + x * BOX_BYTES, &map_v, x * 64, kvh, row, &full_bar[st]);
+                    }
                     ++i;
                 }
         }
@@ -152,146 +170,164 @@ __global__ void __launch_bounds__(kBlock, (HD == 128 || GC == 4) ? 2 : 3) attn_d
     }
     pdl_wait();  // q and the newest cache row come from the kernel before this one
     int pi = 0;  // pages consumed so far (ring position)
+    const uint32_t sw = uint32_t(lane & 7);   // swizzle of the row this lane addresses (rows are taken eight at a time)
 
-    for (int g0 = 0; g0 < G; g0 += GC) {
-        const int gc = min(GC, G - g0);
-        float q[GC][8], acc[GC][8], mi[GC], li[GC];
+    for (int g0 = 0; g0 < G; g0 += kHeads) {
+        const int gc = min(kHeads, G - g0);
+        // A fragments of the scaled queries: row lr = hi part of head lr, row lr + 8 = lo part
+        uint32_t qf[KS][4];
 #pragma unroll
-        for (int g = 0; g < GC; ++g) {
-            mi[g] = -INFINITY; li[g] = 0.f;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) { acc[g][i] = 0.f; q[g][i] = 0.f; }
-            if (g < gc && act) {
-                const float4* qp = reinterpret_cast<const float4*>(a.q + (size_t(b) * a.nq + kvh * G + g0 + g) * HD + sl * 8);
-                float4 x0 = qp[0], x1 = qp[1];
-                q[g][0] = x0.x * p.scale; q[g][1] = x0.y * p.scale; q[g][2] = x0.z * p.scale; q[g][3] = x0.w * p.scale;
-                q[g][4] = x1.x * p.scale; q[g][5] = x1.y * p.scale; q[g][6] = x1.z * p.scale; q[g][7] = x1.w * p.scale;
+        for (int k = 0; k < KS; ++k) {
+            float2 x = make_float2(0.f, 0.f), y = x;
+            if (lr < gc) {
+                const float* qp = a.q + (size_t(b) * a.nq + kvh * G + g0 + lr) * HD + k * 16 + lc;
+                x = *reinterpret_cast<const float2*>(qp);
+                y = *reinterpret_cast<const float2*>(qp + 8);
             }
+            split_h2(x.x * p.scale, x.y * p.scale, qf[k][0], qf[k][1]);
+            split_h2(y.x * p.scale, y.y * p.scale, qf[k][2], qf[k][3]);
         }
+        float o[NV][4], m = -INFINITY, l = 0.f;
+#pragma unroll
+        for (int v = 0; v < NV; ++v)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) o[v][e] = 0.f;
         for (int lp = split; lp < n_pages; lp += a.splits) {
             if (SW && (lp + 1) * FORGE_KV_PAGE <= t_first) continue;  // the whole page lies before the window
-            const int t_page = lp * FORGE_KV_PAGE;
+            const int t0 = lp * FORGE_KV_PAGE + warp * 16;            // the warp's sixteen keys
             const int st = pi % p.stages;
             if (!mbar_wait(&full_bar[st], (pi / p.stages) & 1) && a.err) atomicExch(a.err, 1);
-            const unsigned char* ks = ring + size_t(st) * 2 * PAGE_BYTES;
-            const unsigned char* vs = ks + PAGE_BYTES;
-            for (int base = warp * RPW; base < FORGE_KV_PAGE; base += PARTS * UNR) {
-                uint4 kr[UNR], vr[UNR];
-#pragma unroll
-                for (int u = 0; u < UNR; ++u) {
-                    const int tp = base + u * PARTS + seg;
-                    kr[u] = make_uint4(0, 0, 0, 0);
-                    vr[u] = make_uint4(0, 0, 0, 0);
-                    if (tp < FORGE_KV_PAGE && t_page + tp < n_ctx && (!SW || t_page + tp >= t_first) && act) {
-                        if (t_page + tp == n_ctx - 1) {
-                            // the newest row is being written by the kernel in front while the page is copied: it is
-                            // read from global memory, after the wait
-                            const size_t off = (size_t(seq_base) + size_t(pt ? pt[lp] : lp) * FORGE_KV_PAGE + tp) * kvd + size_t(kvh) * HD + sl * 8;
-                            kr[u] = __ldcg(reinterpret_cast<const uint4*>(a.k_pool + off));
-                            vr[u] = __ldcg(reinterpret_cast<const uint4*>(a.v_pool + off));
-                        } else {
-                            kr[u] = *reinterpret_cast<const uint4*>(ks + size_t(tp) * HD * 2 + sl * 16);
-                            vr[u] = *reinterpret_cast<const uint4*>(vs + size_t(tp) * HD * 2 + sl * 16);
-                        }
+            unsigned char* const ks = ring + size_t(st) * 2 * PAGE_BYTES + warp * 16 * 128;
+            if (t0 < n_ctx && (!SW || t0 + 16 > t_first)) {
+                if (n_ctx - 1 - t0 < 16) {
+                    // the newest row was being written by the kernel in front while the page was copied: it is taken from global memory
+                    const int r = n_ctx - 1 - t0;
+                    if (lane < HD / 4) {
+                        const int c = lane % (HD / 8), which = lane / (HD / 8);
+                        const __half* src = (which ? a.v_pool : a.k_pool) + (seq_base + size_t(pt ? pt[lp] : lp) * FORGE_KV_PAGE + warp * 16 + r) * kvd + size_t(kvh) * HD + c * 8;
+                        *reinterpret_cast<uint4*>(ks + which * PAGE_BYTES + (c >> 3) * BOX_BYTES + r * 128 + (((c & 7) ^ (r & 7)) << 4)) = __ldcg(reinterpret_cast<const uint4*>(src));
                     }
+                    __syncwarp();
                 }
-                // the UNR scores of a head are formed independently, then folded into the running state in one
-                // softmax step (one rescale per group instead of one per position)
-                float sc[UNR][GC];
-#pragma unroll
-                for (int u = 0; u < UNR; ++u) {
-                    float kf[8];
-                    unpack8(kr[u], kf);
-#pragma unroll
-                    for (int g = 0; g < GC; ++g) {
-                        float d = 0.f;
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) d += q[g][i] * kf[i];
-                        sc[u][g] = d;
+                if (n_ctx - t0 < 16 || (SW && t0 < t_first)) {
+                    // a weight of zero must not meet what lies in rows that are not seen (another sequence's, or nothing yet)
+                    for (int i = lane; i < 16 * BOXES * 8; i += 32) {
+                        const int r = i & 15, c = i >> 4;
+                        if (t0 + r >= n_ctx || (SW && t0 + r < t_first)) *reinterpret_cast<uint4*>(ks + PAGE_BYTES + (c >> 3) * BOX_BYTES + r * 128 + ((c & 7) << 4)) = make_uint4(0, 0, 0, 0);
                     }
+                    __syncwarp();
                 }
+                const uint32_t kb = smem_u32(ks), vb = kb + PAGE_BYTES;
+                const uint32_t krow = kb + uint32_t((lane & 7) + ((lane >> 4) << 3)) * 128, vrow = vb + uint32_t(lane & 15) * 128;
+                float s[2][2][4];   // [key tile][even and odd steps][fragment]
 #pragma unroll
-                for (int o = W / 2; o > 0; o >>= 1)
+                for (int e = 0; e < 16; ++e) s[e >> 3][(e >> 2) & 1][e & 3] = 0.f;
 #pragma unroll
-                    for (int u = 0; u < UNR; ++u)
-#pragma unroll
-                        for (int g = 0; g < GC; ++g) sc[u][g] += __shfl_xor_sync(0xffffffffu, sc[u][g], o);
-#pragma unroll
-                for (int u = 0; u < UNR; ++u) {
-                    const int tp = base + u * PARTS + seg;
-                    if (!(tp < FORGE_KV_PAGE && t_page + tp < n_ctx && (!SW || t_page + tp >= t_first))) {
-#pragma unroll
-                        for (int g = 0; g < GC; ++g) sc[u][g] = -INFINITY;
-                    }
+                for (int k = 0; k < KS; ++k) {
+                    uint32_t f[4];
+                    const uint32_t c = uint32_t(2 * k + ((lane >> 3) & 1));   // 16-byte piece of the row
+                    ldsm4(f, krow + (c >> 3) * BOX_BYTES + (((c & 7) ^ sw) << 4));
+                    mma16(s[0][k & 1], qf[k], f[0], f[1]);
+                    mma16(s[1][k & 1], qf[k], f[2], f[3]);
                 }
-                float vf[UNR][8];
+                float sc[4];
 #pragma unroll
-                for (int u = 0; u < UNR; ++u) unpack8(vr[u], vf[u]);
+                for (int j = 0; j < 4; ++j) {
+                    const int t = j >> 1, e = j & 1, key = t0 + t * 8 + lc + e;
+                    sc[j] = (s[t][0][e] + s[t][1][e]) + (s[t][0][e + 2] + s[t][1][e + 2]);
+                    if (key >= n_ctx || (SW && key < t_first)) sc[j] = -INFINITY;
+                }
+                float mn = fmaxf(fmaxf(sc[0], sc[1]), fmaxf(sc[2], sc[3]));
+                mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 1));
+                mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 2));
+                mn = fmaxf(mn, m);
+                const float at = mn == -INFINITY ? 0.f : mn, es = exp2f(m - at);   // a tile holds a visible key, but its score may be -inf
+                float pr[4];
 #pragma unroll
-                for (int g = 0; g < GC; ++g) {
-                    float mn = mi[g];
+                for (int j = 0; j < 4; ++j) pr[j] = exp2f(sc[j] - at);
+                m = mn;
+                l = l * es + ((pr[0] + pr[1]) + (pr[2] + pr[3]));
+                uint32_t pf[4];
+                split_h2(pr[0], pr[1], pf[0], pf[1]);
+                split_h2(pr[2], pr[3], pf[2], pf[3]);
 #pragma unroll
-                    for (int u = 0; u < UNR; ++u) mn = fmaxf(mn, sc[u][g]);
-                    if (mn == -INFINITY || g >= gc) continue;
-                    const float es = exp_rel(mi[g], mn);
-                    float pr[UNR], ps = 0.f;
+                for (int v = 0; v < NV; ++v)
 #pragma unroll
-                    for (int u = 0; u < UNR; ++u) { pr[u] = exp_rel(sc[u][g], mn); ps += pr[u]; }
-                    mi[g] = mn;
-                    li[g] = li[g] * es + ps;
+                    for (int e = 0; e < 4; ++e) o[v][e] *= es;
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        float t = acc[g][i] * es;
-#pragma unroll
-                        for (int u = 0; u < UNR; ++u) t += pr[u] * vf[u][i];
-                        acc[g][i] = t;
-                    }
+                for (int v = 0; v < NV; v += 2) {
+                    uint32_t f[4];
+                    const uint32_t c = uint32_t(v + (lane >> 4));
+                    ldsm4t(f, vrow + (c >> 3) * BOX_BYTES + (((c & 7) ^ sw) << 4));
+                    mma16(o[v], pf, f[0], f[1]);
+                    mma16(o[v + 1], pf, f[2], f[3]);
                 }
             }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // this warp may have written a row of the page
             __syncwarp();
             if (lane == 0) mbar_arrive(&empty_bar[st]);
             ++pi;
         }
-        // ---- merge the CTA's parts: weights once per (part, head), then one weighted sum per output
-        csync();
+        // ---- the warps' parts become the CTA's
+        l += __shfl_xor_sync(0xffffffffu, l, 1);
+        l += __shfl_xor_sync(0xffffffffu, l, 2);
+        if (lc == 0) { s_ml[warp][lr][0] = m; s_ml[warp][lr][1] = l; }
 #pragma unroll
-        for (int g = 0; g < GC; ++g) {
-            if (sl == 0) { s_m[part][g] = mi[g]; s_l[part][g] = li[g]; }
-            if (act) {
-                *reinterpret_cast<float4*>(&s_acc[part][g][sl * 8]) = make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]);
-                *reinterpret_cast<float4*>(&s_acc[part][g][sl * 8 + 4]) = make_float4(acc[g][4], acc[g][5], acc[g][6], acc[g][7]);
-            }
-        }
-        csync();
-        if (threadIdx.x < PARTS * GC) {
-            const int pp = threadIdx.x % PARTS, g = threadIdx.x / PARTS;
-            float M = -INFINITY;
-#pragma unroll
-            for (int j = 0; j < PARTS; ++j) M = fmaxf(M, s_m[j][g]);
-            s_w[pp][g] = exp_rel(s_m[pp][g], M);
-        }
+        for (int v = 0; v < NV; ++v)
+            *reinterpret_cast<float2*>(s_acc + (warp * kHeads + lr) * HD + v * 8 + lc) = make_float2(o[v][0] + o[v][2], o[v][1] + o[v][3]);
         csync();
         for (int idx = threadIdx.x; idx < gc * HD; idx += kThreads) {
-            const int g = idx / HD, dd = idx % HD;
-            float A = 0.f;
+            const int g = idx / HD;
+            float M = -INFINITY, A = 0.f, L = 0.f;
 #pragma unroll
-            for (int pp = 0; pp < PARTS; ++pp) A += s_acc[pp][g][dd] * s_w[pp][g];
-            const int head = kvh * G + g0 + g;
-            float M = -INFINITY, L = 0.f;
-            if (dd == 0 || a.splits == 1) {
+            for (int w = 0; w < 4; ++w) M = fmaxf(M, s_ml[w][g][0]);
 #pragma unroll
-                for (int pp = 0; pp < PARTS; ++pp) { M = fmaxf(M, s_m[pp][g]); L += s_l[pp][g] * s_w[pp][g]; }
+            for (int w = 0; w < 4; ++w) {
+                const float f = exp2_rel(s_ml[w][g][0], M);
+                A += s_acc[w * kHeads * HD + idx] * f;
+                L += s_ml[w][g][1] * f;
             }
             if (a.splits == 1) {
-                store_out(a, (size_t(b) * a.nq + head) * HD + dd, A * (1.0f / L));
+                store_out(a, (size_t(b) * a.nq + kvh * G + g0) * HD + idx, A * (1.0f / L));
+            } else if (CL) {
+                s_acc[idx] = A;   // over warp 0's own value
+                if (idx % HD == 0) { s_cml[g][0] = M; s_cml[g][1] = L; }
             } else {
-                float* w = a.ws + ((size_t(b) * a.nq + head) * a.splits + split) * (HD + 2);
-                w[2 + dd] = A;
-                if (dd == 0) { w[0] = M; w[1] = L; }
+                float* w = a.ws + ((size_t(b) * a.nq + kvh * G + g0 + g) * a.splits + split) * (HD + 2);
+                w[2 + idx % HD] = A;
+                if (idx % HD == 0) { w[0] = M; w[1] = L; }
             }
         }
+        if (CL && a.splits > 1) {
+            // ---- the CTAs' parts become the result, each CTA finishing a share of it
+            cluster_sync();
+            const int items = gc * HD, share = (items + a.splits - 1) / a.splits;
+            for (int idx = split * share + threadIdx.x; idx < min(items, (split + 1) * share); idx += kThreads) {
+                const int g = idx / HD;
+                float pm[kClusterSplits], pl[kClusterSplits], px[kClusterSplits], M = -INFINITY, A = 0.f, L = 0.f;
+#pragma unroll
+                for (int s = 0; s < kClusterSplits; ++s) {
+                    const bool on = s < a.splits;
+                    pm[s] = on ? remote_f32(cluster_addr(&s_cml[g][0], s)) : -INFINITY;
+                    pl[s] = on ? remote_f32(cluster_addr(&s_cml[g][1], s)) : 0.f;
+                    px[s] = on ? remote_f32(cluster_addr(s_acc + idx, s)) : 0.f;
+                }
+#pragma unroll
+                for (int s = 0; s < kClusterSplits; ++s) M = fmaxf(M, pm[s]);
+#pragma unroll
+                for (int s = 0; s < kClusterSplits; ++s) {
+                    const float f = exp2_rel(pm[s], M);
+                    A += px[s] * f;
+                    L += pl[s] * f;
+                }
+                store_out(a, (size_t(b) * a.nq + kvh * G + g0) * HD + idx, A * (1.0f / L));
+            }
+            cluster_sync();   // nobody leaves, or starts the next heads, while its sums are read
+        } else {
+            csync();
+        }
     }
-    if (a.splits == 1) return;
+    if (CL || a.splits == 1) return;
 
     // ---- last CTA of this (batch, kv head) merges the splits
     __threadfence();
@@ -304,87 +340,68 @@ __global__ void __launch_bounds__(kBlock, (HD == 128 || GC == 4) ? 2 : 3) attn_d
     csync();
     if (!s_last) return;
     __threadfence();
-    // One round trip: every thread first issues the loads of its two output columns from all splits, then the
-    // warps turn the splits' (max, sum) pairs into normalised weights (lane = split), then the weighted sums.
     const float* ws_kvh = a.ws + (size_t(b) * a.nq + size_t(kvh) * G) * a.splits * (HD + 2);
-    const int nout2 = G * HD / 2;
-    for (int i0 = 0; i0 < nout2; i0 += kThreads) {
-        const int idx = i0 + threadIdx.x;
-        const bool on = idx < nout2;
-        const int g = on ? idx / (HD / 2) : 0, d2 = on ? idx % (HD / 2) : 0;
-        const float* w0 = ws_kvh + size_t(g) * a.splits * (HD + 2) + 2 + 2 * d2;
-        float2 pa[kMaxSplits];
+    for (int g = warp; g < G; g += kThreads / 32) {
+        const float* w = ws_kvh + (size_t(g) * a.splits + lane) * (HD + 2);
+        const float m = lane < a.splits ? __ldcg(w) : -INFINITY;
+        const float l = lane < a.splits ? __ldcg(w + 1) : 0.f;
+        float M = m;
 #pragma unroll
-        for (int s = 0; s < kMaxSplits; ++s)
-            pa[s] = (on && s < a.splits) ? __ldcg(reinterpret_cast<const float2*>(w0 + size_t(s) * (HD + 2))) : make_float2(0.f, 0.f);
-        if (i0 == 0) {
-            for (int g2 = warp; g2 < G; g2 += kThreads / 32) {
-                const float* w = ws_kvh + (size_t(g2) * a.splits + lane) * (HD + 2);
-                const float m = lane < a.splits ? __ldcg(w) : -INFINITY;
-                const float l = lane < a.splits ? __ldcg(w + 1) : 0.f;
-                float M = m;
+        for (int x = 16; x > 0; x >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, x));
+        const float wt = exp2_rel(m, M);
+        float L = l * wt;
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
-                const float wt = exp_rel(m, M);
-                float L = l * wt;
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
-                s_fw[lane][g2] = wt * (1.0f / L);
-            }
-            csync();
-        }
-        float2 A = make_float2(0.f, 0.f);
-#pragma unroll
-        for (int s = 0; s < kMaxSplits; ++s) {
-            const float wt = s < a.splits ? s_fw[s][g] : 0.f;
-            A.x += pa[s].x * wt;
-            A.y += pa[s].y * wt;
-        }
-        if (on) store_out2(a, (size_t(b) * a.nq + kvh * G + g) * HD + 2 * d2, A);
+        for (int x = 16; x > 0; x >>= 1) L += __shfl_xor_sync(0xffffffffu, L, x);
+        s_fw[lane][g] = wt * (1.0f / L);
+    }
+    csync();
+    for (int idx = threadIdx.x; idx < G * HD; idx += kThreads) {
+        const int g = idx / HD;
+        const float* w0 = ws_kvh + size_t(g) * a.splits * (HD + 2) + 2 + idx % HD;
+        float A = 0.f;
+#pragma unroll 8
+        for (int s = 0; s < a.splits; ++s) A += __ldcg(w0 + size_t(s) * (HD + 2)) * s_fw[s][g];
+        store_out(a, (size_t(b) * a.nq + kvh * G) * HD + idx, A);
     }
 }
 
 }  // namespace
 
-int attn_decode_splits(int pages, int groups, int sms, int hd, int heads_per_group) {
-    // CTAs run in rounds over the resident slots (three CTAs per SM; two with 128-wide heads or four query heads per pass):
-    // pick the split count whose rounds waste the least, a CTA's work being 1 / splits of a sequence plus a few per cent
-    // per extra split for the merge.  Never more splits than pages.
-    const int per_sm = (hd == 128 || heads_per_group >= 3) ? 2 : 3;
+// Context splits for `groups` = batch * kv_heads independent (sequence, KV head) pairs over `pages` pages.  CTAs run in rounds over the resident slots; a
+// CTA costs a fixed share (query, merge) and a share per page, so the splits are those whose rounds are done first: one sequence takes
+// eight, sixteen sequences of 32 KV heads one.  More than a cluster's eight only where a CTA would still walk sixteen pages.
+int attn_decode_splits(int pages, int groups, int sms, int hd, int) {
+    const int per_sm = hd == 64 ? 3 : 2;
     const long slots = long(sms) * per_sm;
-    const int smax = std::max(1, std::min(pages, kMaxSplits));
+    const int top = pages > 16 * kClusterSplits ? kMaxSplits : kClusterSplits, smax = std::max(1, std::min(pages, top));
+    const double page = hd == 64 ? 0.3 : 0.5, fixed = 1.5;
     int best = 1;
     double best_cost = 1e30;
     for (int s = 1; s <= smax; ++s) {
         const long rounds = (long(groups) * s + slots - 1) / slots;
-        const double cost = double(rounds) / s * (1.0 + 0.03 * (s - 1));
+        const double cost = double(rounds) * (fixed + (s > 1 ? 0.5 : 0.0) + (s > kClusterSplits ? 1.0 : 0.0) + page * ((pages + s - 1) / s));
         if (cost < best_cost - 1e-12) { best_cost = cost; best = s; }
     }
     return best;
 }
 
-size_t attn_decode_ws_floats(int batch, int nq, int hd, int splits) { return size_t(batch) * nq * splits * (hd + 2); }
+// workspace of the splits that are merged through global memory (0: none is needed)
+size_t attn_decode_ws_floats(int batch, int nq, int hd, int splits) { return splits > kClusterSplits ? size_t(batch) * nq * splits * (hd + 2) : 0; }
 
-template <int HD, bool SW, int GC>
+template <int HD, bool SW>
 int32_t launch_decode(const CUtensorMap& mk, const CUtensorMap& mv, const DecParams& p, dim3 grid, cudaStream_t st) {
-    const size_t smem = size_t(p.stages) * 2 * FORGE_KV_PAGE * HD * 2;
-    auto kern = attn_decode_kernel<HD, SW, GC>;
-    FORGE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(size_t(kStages) * 2 * FORGE_KV_PAGE * HD * 2)));
-    FORGE_CUDA(launch_pdl(kern, grid, dim3(kBlock), smem, st, mk, mv, p));
+    constexpr int kPage = (HD + 63) / 64 * FORGE_KV_PAGE * 128, kSums = 4 * kHeads * HD * 4;
+    const size_t smem = size_t(p.stages) * 2 * kPage + kSums + 1024;
+    auto kern = p.a.splits <= kClusterSplits ? attn_decode_kernel<HD, SW, true> : attn_decode_kernel<HD, SW, false>;
+    FORGE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kStages * 2 * kPage + kSums + 1024));
+    FORGE_CUDA(launch_pdl_cluster(kern, grid, dim3(kBlock), p.a.splits <= kClusterSplits ? p.a.splits : 1, smem, st, mk, mv, p));
     FORGE_LAUNCH_CHECK();
     return FORGE_OK;
 }
 
-template <int GC>
-int32_t launch_decode_hd(int hd, bool sw, const CUtensorMap& mk, const CUtensorMap& mv, const DecParams& p, dim3 grid, cudaStream_t st) {
-    if (hd == 64) return sw ? launch_decode<64, true, GC>(mk, mv, p, grid, st) : launch_decode<64, false, GC>(mk, mv, p, grid, st);
-    if (hd == 96) return sw ? launch_decode<96, true, GC>(mk, mv, p, grid, st) : launch_decode<96, false, GC>(mk, mv, p, grid, st);
-    return sw ? launch_decode<128, true, GC>(mk, mv, p, grid, st) : launch_decode<128, false, GC>(mk, mv, p, grid, st);
-}
-
 int32_t attn_decode(const AttnDecodeArgs& a, cudaStream_t st) {
     if (a.nq % a.nkv) { set_error("attention: num_heads %d not a multiple of num_kv_heads %d", a.nq, a.nkv); return FORGE_ERR_SHAPE; }
-    if (a.splits < 1 || (a.splits > 1 && (!a.ws || !a.counters))) { set_error("attention: split workspace missing"); return FORGE_ERR_INVALID_ARG; }
+    if (a.splits < 1 || (a.splits > kClusterSplits && (!a.ws || !a.counters))) { set_error("attention: split workspace missing"); return FORGE_ERR_INVALID_ARG; }
     if (a.nq / a.nkv > kMaxGroup) { set_error("attention: at most %d query heads per KV head", kMaxGroup); return FORGE_ERR_SHAPE; }
     if (a.splits > kMaxSplits) { set_error("attention: at most %d context splits", kMaxSplits); return FORGE_ERR_INVALID_ARG; }
     if (a.hd != 64 && a.hd != 96 && a.hd != 128) { set_error("attention: head_dim %d unsupported (64, 96, 128)", a.hd); return FORGE_ERR_SHAPE; }
@@ -399,18 +416,15 @@ int32_t attn_decode(const AttnDecodeArgs& a, cudaStream_t st) {
         FORGE_TRY(make_kv_map(&mk, a.k_pool, a.hd, a.nkv, rows));
         FORGE_TRY(make_kv_map(&mv, a.v_pool, a.hd, a.nkv, rows));
     }
-    // ring depth: the pages a CTA will see (per pass over the query heads), at most kStages
+    // ring depth: the pages a CTA will see, at most what lets three CTAs (two with wider heads) share an SM
     const int ctx = a.seq_len ? a.max_ctx : a.seq_len_host;
     const int pages_per_cta = ((ctx + FORGE_KV_PAGE - 1) / FORGE_KV_PAGE + a.splits - 1) / a.splits;
-    // three CTAs per SM (two with 128-wide heads) share its shared memory with their merge buffers: a ring of 48 KB
-    // each for 64- and 96-wide heads (3 and 2 pages of K and V), 64 KB (2 pages) for 128-wide
-    const int fit = std::max(2, int((56u << 10) / (2u * FORGE_KV_PAGE * a.hd * sizeof(__half))));
-    DecParams p{a, 1.0f / sqrtf(float(a.hd)), pages_per_cta <= 2 ? 2 : std::min(kStages, fit)};
+    DecParams p{a, kLog2e / sqrtf(float(a.hd)), std::max(1, std::min(pages_per_cta, a.hd == 64 ? 4 : 2))};
     dim3 grid(a.splits, a.nkv, a.batch);
-    const int group = a.nq / a.nkv;
-    if (group == 1) return launch_decode_hd<1>(a.hd, a.window > 0, mk, mv, p, grid, st);
-    if (group == 2) return launch_decode_hd<2>(a.hd, a.window > 0, mk, mv, p, grid, st);
-    return launch_decode_hd<4>(a.hd, a.window > 0, mk, mv, p, grid, st);
+    const bool sw = a.window > 0;
+    if (a.hd == 64) return sw ? launch_decode<64, true>(mk, mv, p, grid, st) : launch_decode<64, false>(mk, mv, p, grid, st);
+    if (a.hd == 96) return sw ? launch_decode<96, true>(mk, mv, p, grid, st) : launch_decode<96, false>(mk, mv, p, grid, st);
+    return sw ? launch_decode<128, true>(mk, mv, p, grid, st) : launch_decode<128, false>(mk, mv, p, grid, st);
 }
 
 }  // namespace forge

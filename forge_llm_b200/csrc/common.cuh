@@ -267,11 +267,12 @@ struct AttnDecodeArgs {
     // instead of f32 `out`
     __half* out16 = nullptr; __half* out16_lo = nullptr;
 };
-// context splits for `groups` = batch * kv_heads independent (sequence, KV head) pairs over `pages` pages
+// context splits for `groups` = batch * kv_heads independent (sequence, KV head) pairs over `pages` pages.  Up to eight need no
+// workspace (attn_decode_ws_floats is 0): a.ws and a.counters may then be null
 int attn_decode_splits(int pages, int groups, int sms, int hd, int heads_per_group);
 size_t attn_decode_ws_floats(int batch, int nq, int hd, int splits);
 // Tiled tensor map over an fp16 K or V pool of `rows` rows of kv_heads * head_dim values: dimensions {head_dim, kv_heads,
-// rows}, box {head_dim, 1, 64} = one page of one KV head (`out`: a CUtensorMap in host memory)
+// rows}, box {64, 1, 64} = 64 dimensions of one page of one KV head, SWIZZLE_128B (`out`: a CUtensorMap in host memory)
 int32_t make_kv_map(void* out, const __half* pool, int head_dim, int kv_heads, size_t rows);
 int32_t attn_decode(const AttnDecodeArgs& a, cudaStream_t st);
 
