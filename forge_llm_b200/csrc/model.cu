@@ -328,7 +328,6 @@ struct PrefillToken { int seq; const uint32_t* tok; bool head; float* trace_dst;
 // order this follows).  Activations are packed as fp16 hi/lo fragments in front of each product (with the RMSNorm or
 // SiLU*up that feeds it), bias + RoPE + cache append and the single-query attention run per sequence.
 constexpr int kBatchGroup = 16;
-int32_t ensure_batch_buffers(ForgeModel* m) {
 // splits of the decode attention for the sequences of one launch; the workspace of more than eight was made for all of the cache's
 int launch_splits(const ForgeModel* m, const ForgeKV* kv, int batch) {
     if (batch >= kv->batch) return kv->splits;
@@ -337,6 +336,7 @@ int launch_splits(const ForgeModel* m, const ForgeKV* kv, int batch) {
     const int s = attn_decode_splits(kv->pages_per_seq, batch * m->nkv, sms, m->hd, m->nq / m->nkv);
     return attn_decode_ws_floats(1, 1, 1, s) ? kv->splits : s;
 }
+int32_t ensure_batch_buffers(ForgeModel* m) {
     if (m->d_bact) return FORGE_OK;
     const int maxK = std::max({m->h, m->qk, m->ff});
     FORGE_TRY(dev_alloc(m, &m->d_bact, gemv_batch_act_words(maxK, kBatchGroup)));
