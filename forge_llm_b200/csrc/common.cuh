@@ -238,7 +238,10 @@ int32_t qkv_post_rows(const float* qkv, int batch, const float* bias, const floa
 int32_t argmax_last(uint32_t* result, const float* logits, int n, int batch, cudaStream_t st);
 // many-CTA form; sval/sidx: [batch][kArgmaxSlices] scratch, ticket: [batch] zero-initialised counters
 constexpr int kArgmaxSlices = 148;
-int32_t argmax_slices(uint32_t* result, const float* logits, int n, int batch, float* sval, int* sidx, int* ticket, cudaStream_t st);
+// adv.seq_len != null: the step's bookkeeping (step_advance) rides along
+struct StepAdvance { int32_t* seq_len; int32_t* step; uint32_t* extra; };
+int32_t argmax_slices(uint32_t* result, const float* logits, int n, int batch, float* sval, int* sidx, int* ticket, cudaStream_t st,
+                      StepAdvance adv = {nullptr, nullptr, nullptr});
 int32_t f32_to_f16(__half* out, __half* lo, const float* in, size_t n, cudaStream_t st);
 // In place: the rows (hi + lo) become their Q8_0 form q * f16(scale) per 32 values (emit.rs:1412-1440), the input of
 // every K-quant product, again split into hi + lo (exact: an 8-bit integer times an f16).

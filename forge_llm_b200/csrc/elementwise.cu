@@ -160,6 +160,7 @@ __global__ void residual_add_kernel(float* a, const float* b, size_t n) {
 }
 
 __global__ void embedding_kernel(float* out, const float* table, const uint32_t* tokens, int h, uint32_t* hist, const int32_t* step) {
+    pdl_trigger();
     if (hist && threadIdx.x == 0) hist[size_t(*step) * gridDim.x + blockIdx.x] = tokens[blockIdx.x];
     const float4* src = reinterpret_cast<const float4*>(table + size_t(tokens[blockIdx.x]) * h);
     float4* dst = reinterpret_cast<float4*>(out + size_t(blockIdx.x) * h);
@@ -350,7 +351,9 @@ __global__ void argmax_kernel(uint32_t* result, const float* logits, int n) {
 
 // Two-stage variant for large vocabularies: every CTA scans a slice, the last CTA to finish (atomic
 // ticket) reduces the per-CTA winners with the same tie rule.  scratch: [batch][gridDim.x] pairs.
-__global__ void argmax_slices_kernel(uint32_t* result, const float* logits, int n, float* sval, int* sidx, int* ticket) {
+// `adv`: the same thread also moves the sequence on (a step's last kernel; nothing of the step is running any more).
+__global__ void argmax_slices_kernel(uint32_t* result, const float* logits, int n, float* sval, int* sidx, int* ticket, StepAdvance adv) {
+    pdl_wait();
     __shared__ float bv[32];
     __shared__ int bi[32];
     __shared__ int s_last;
@@ -360,9 +363,16 @@ __global__ void argmax_slices_kernel(uint32_t* result, const float* logits, int 
     float best = -INFINITY;
     int idx = -1;
     auto better = [](float v, int i, float bv_, int bi_) { return i >= 0 && (bi_ < 0 || v > bv_ || (v == bv_ && i > bi_)); };
-    for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-        float v = x[i];
-        if (better(v, i, best, idx)) { best = v; idx = i; }
+    constexpr int kAhead = 8;   // loads in flight per thread
+    for (int i0 = lo + threadIdx.x; i0 < hi; i0 += kAhead * blockDim.x) {
+        float v[kAhead];
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j) v[j] = i0 + j * int(blockDim.x) < hi ? x[i0 + j * blockDim.x] : 0.f;
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j) {
+            const int i = i0 + j * blockDim.x;
+            if (i < hi && better(v[j], i, best, idx)) { best = v[j]; idx = i; }
+        }
     }
     auto block_reduce = [&]() {
 #pragma unroll
@@ -399,7 +409,12 @@ __global__ void argmax_slices_kernel(uint32_t* result, const float* logits, int 
         if (better(v, vi, best, idx)) { best = v; idx = vi; }
     }
     block_reduce();
-    if (threadIdx.x == 0) result[b] = uint32_t(idx < 0 ? 0 : idx);
+    if (threadIdx.x == 0) {
+        result[b] = uint32_t(idx < 0 ? 0 : idx);
+        if (adv.seq_len) adv.seq_len[b] += 1;
+        if (b == 0 && adv.step) *adv.step += 1;
+        if (b == 0 && adv.extra) *adv.extra += 1;
+    }
 }
 
 __global__ void f32_to_f16_kernel(__half* out, __half* lo, const float* in, size_t n) {
@@ -432,6 +447,7 @@ __global__ void __launch_bounds__(1024) token_nll_kernel(double* out, const floa
 }
 
 __global__ void step_advance_kernel(int32_t* seq_len, int batch, int32_t* step, uint32_t* extra_counter) {
+    pdl_wait();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < batch) seq_len[i] += 1;
     if (i == 0 && step) *step += 1;
@@ -541,9 +557,11 @@ int32_t argmax_last(uint32_t* result, const float* logits, int n, int batch, cud
     FORGE_LAUNCH_CHECK();
     return FORGE_OK;
 }
-int32_t argmax_slices(uint32_t* result, const float* logits, int n, int batch, float* sval, int* sidx, int* ticket, cudaStream_t st) {
-    dim3 grid(kArgmaxSlices, batch);
-    argmax_slices_kernel<<<grid, 256, 0, st>>>(result, logits, n, sval, sidx, ticket);
+int32_t argmax_slices(uint32_t* result, const float* logits, int n, int batch, float* sval, int* sidx, int* ticket, cudaStream_t st, StepAdvance adv) {
+    // one row is spread over all SMs; with more rows a slice is longer, four CTAs per SM altogether (148 slices for each of 64 rows of
+    // 151936 logits: 40 us, the fences and tickets of 9472 CTAs)
+    const int slices = std::max(1, std::min(kArgmaxSlices, 4 * kArgmaxSlices / batch));
+    FORGE_CUDA(launch_pdl(argmax_slices_kernel, dim3(slices, batch), dim3(256), 0, st, result, logits, n, sval, sidx, ticket, adv));
     FORGE_LAUNCH_CHECK();
     return FORGE_OK;
 }
@@ -603,7 +621,7 @@ int32_t token_nll(double* out, const float* logits, int n, uint32_t target, cuda
     return FORGE_OK;
 }
 int32_t step_advance(int32_t* seq_len, int batch, int32_t* step, cudaStream_t st, uint32_t* extra_counter) {
-    step_advance_kernel<<<(batch + 127) / 128, 128, 0, st>>>(seq_len, batch, step, extra_counter);
+    FORGE_CUDA(launch_pdl(step_advance_kernel, dim3((batch + 127) / 128), dim3(128), 0, st, seq_len, batch, step, extra_counter));
     FORGE_LAUNCH_CHECK();
     return FORGE_OK;
 }

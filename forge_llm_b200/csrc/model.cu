@@ -435,7 +435,7 @@ int32_t decode_launches_batched(ForgeModel* m, ForgeKV* kv, int batch, bool gree
         FORGE_TRY(batched_row_sliced(m, L.down_t, m->p_gu, size_t(2) * m->ff, SILU, n, &sums, &pending, st));
     }
     FORGE_TRY(normed_product(m->lm_head_t, m->final_norm, m->d_logits));
-    if (greedy) FORGE_TRY(argmax_slices(m->d_tok, m->d_logits, m->V, n, m->d_amax_val, m->d_amax_idx, m->d_amax_ticket, st));
+    if (greedy) return argmax_slices(m->d_tok, m->d_logits, m->V, n, m->d_amax_val, m->d_amax_idx, m->d_amax_ticket, st, {kv->d_seq_len, m->d_step, sums ? m->d_tpx_step : nullptr});
     return step_advance(kv->d_seq_len, n, m->d_step, st, sums ? m->d_tpx_step : nullptr);
 }
 
@@ -475,7 +475,7 @@ int32_t decode_launches_gemm(ForgeModel* m, ForgeKV* kv, int batch, bool greedy,
         FORGE_TRY(row_sliced_gemm_norm(m, L.down, m->p_act16, flo, n, l + 1 < c.num_layers ? m->layers[l + 1].attn_norm : m->final_norm, nlo, st));
     }
     FORGE_TRY(gemm_f16a(m->d_logits, m->p_normed, nlo, m->lm_head, n, nullptr, m->d_err, st));
-    if (greedy) FORGE_TRY(argmax_slices(m->d_tok, m->d_logits, m->V, n, m->d_amax_val, m->d_amax_idx, m->d_amax_ticket, st));
+    if (greedy) return argmax_slices(m->d_tok, m->d_logits, m->V, n, m->d_amax_val, m->d_amax_idx, m->d_amax_ticket, st, {kv->d_seq_len, m->d_step, nullptr});
     return step_advance(kv->d_seq_len, n, m->d_step, st, nullptr);
 }
 
@@ -572,8 +572,9 @@ int32_t decode_launches(ForgeModel* m, ForgeKV* kv, int batch, bool greedy, bool
         if (px) tp_consume(lm);
         FORGE_TRY(gemv_tc(m->lm_head_t, EPI_STORE, lm, m->split, m->d_err, st));
     }
-    if (greedy) FORGE_TRY(argmax_slices(m->d_tok, m->d_logits, m->V, batch, m->d_amax_val, m->d_amax_idx, m->d_amax_ticket, st));
-    FORGE_TRY(step_advance(seq_len, batch, pt ? nullptr : m->d_step, st, px ? m->d_tpx_step : nullptr));
+    const StepAdvance adv{seq_len, pt ? nullptr : m->d_step, px ? m->d_tpx_step : nullptr};
+    if (greedy) FORGE_TRY(argmax_slices(m->d_tok, m->d_logits, m->V, batch, m->d_amax_val, m->d_amax_idx, m->d_amax_ticket, st, adv));
+    else FORGE_TRY(step_advance(adv.seq_len, batch, adv.step, st, adv.extra));
     return FORGE_OK;
 }
 

@@ -1523,7 +1523,7 @@ int32_t stack_decode_launches(ForgeModel* m, ForgeKV* kv, int batch, bool greedy
     if (m->trace_on) { s.trace = m->trace; s.trace_stride = size_t(batch) * S.spec.width; }
     FORGE_TRY(Sequence(m, kv, s).run());
     FORGE_TRY(run_head(m, S.h.p, nullptr, batch, batch, m->d_logits));
-    if (greedy) FORGE_TRY(argmax_slices(m->d_tok, m->d_logits, m->V, batch, m->d_amax_val, m->d_amax_idx, m->d_amax_ticket, m->stream));
+    if (greedy) return argmax_slices(m->d_tok, m->d_logits, m->V, batch, m->d_amax_val, m->d_amax_idx, m->d_amax_ticket, m->stream, {kv->d_seq_len, m->d_step, nullptr});
     return step_advance(kv->d_seq_len, batch, m->d_step, m->stream);
 }
 
