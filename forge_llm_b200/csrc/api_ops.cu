@@ -3,6 +3,7 @@
 // into the kernels' aligned layout in stream-ordered scratch memory, so these are meant for
 // parity tests and one-off use; the session API (forge_model_create) packs weights once.
 #include <cmath>
+#include <mutex>
 #include <vector>
 
 #include "common.cuh"
@@ -11,10 +12,49 @@ using namespace forge;
 
 namespace {
 
+// Scratch of the operator calls comes from a stream-ordered pool of this library's own.  The default pool gives memory back at every
+// synchronisation, and mapping it again cost a caller who waits for each call 0.5 ms for eight products; this one keeps up to kPoolKeep bytes per device
+// until the last packed projection is destroyed.  The pool itself orders reuse between streams and threads.
+constexpr uint64_t kPoolKeep = 256ull << 20;
+constexpr int kMaxDevices = 64;
+std::mutex g_pool_mutex;
+cudaMemPool_t g_pool[kMaxDevices] = {};
+int g_packed_live = 0;
+
+cudaError_t scratch_pool(cudaMemPool_t* out) {
+    int dev = 0;
+    if (cudaError_t e = cudaGetDevice(&dev)) return e;
+    if (dev >= kMaxDevices) return cudaDeviceGetDefaultMemPool(out, dev);
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    if (!g_pool[dev]) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool = nullptr;
+        if (cudaError_t e = cudaMemPoolCreate(&pool, &props)) return e;
+        uint64_t keep = kPoolKeep;
+        if (cudaError_t e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep)) { cudaMemPoolDestroy(pool); return e; }
+        g_pool[dev] = pool;
+    }
+    *out = g_pool[dev];
+    return cudaSuccess;
+}
+void count_packed(int by) {
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    g_packed_live += by;
+    if (g_packed_live == 0)
+        for (cudaMemPool_t p : g_pool) if (p) cudaMemPoolTrimTo(p, 0);   // what is in use stays
+}
+
 struct AsyncBuf {
     void* p = nullptr; cudaStream_t st;
     explicit AsyncBuf(cudaStream_t s) : st(s) {}
-    cudaError_t alloc(size_t bytes) { return cudaMallocAsync(&p, bytes ? bytes : 1, st); }
+    cudaError_t alloc(size_t bytes) {
+        cudaMemPool_t pool = nullptr;
+        if (cudaError_t e = scratch_pool(&pool)) return e;
+        return cudaMallocFromPoolAsync(&p, bytes ? bytes : 1, pool, st);
+    }
     ~AsyncBuf() { if (p) cudaFreeAsync(p, st); }
 };
 
@@ -157,11 +197,16 @@ int32_t forge_packed_create(int32_t quant, const uint8_t* w, int32_t K, int32_t 
     ForgePacked* pk = new ForgePacked();
     int32_t rc = packed_build(quant, w, K, N, static_cast<cudaStream_t>(stream), pk);
     if (rc != FORGE_OK) { packed_free(pk); return rc; }
+    count_packed(1);
     *out = pk;
     return FORGE_OK;
 }
 
-void forge_packed_destroy(ForgePacked* pk) { packed_free(pk); }
+void forge_packed_destroy(ForgePacked* pk) {
+    if (!pk) return;
+    packed_free(pk);
+    count_packed(-1);
+}
 
 int32_t forge_matmul_mat_packed(float* out, int32_t m, const float* in, const ForgePacked* w, void* stream) {
     FORGE_TRY(need_device());
