@@ -112,36 +112,42 @@ __global__ void __launch_bounds__(BOUND ? 320 : 192, COLS <= 256 ? 2 : 1) attn_p
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            bool ok = mbar_wait(&q_full, 0, &s_err);
+        {   // the whole warp runs the loop, one elected lane issues
+            bool ok = all_lanes(mbar_wait(&q_full, 0, &s_err));
             const uint32_t q_base = smem_u32(sQ);
             const int ks = (d.dim + 15) / 16, rs = (d.rot + 15) / 16;   // sixteen-wide steps that hold anything
             auto issue_s = [&](int j) {
                 const uint32_t k_base = smem_u32(sKV + size_t(j % KVS) * stage_bytes);
-                for (int i = 0; i < ks + rs; ++i) {
-                    const int step = i < ks ? i : kch * 4 + (i - ks);
-                    const uint32_t off = uint32_t(step / 4), in = uint32_t((step % 4) * 32);
-                    umma_ss(tmem + kColS, desc_kmajor(q_base + off * Q_CHUNK + in), desc_kmajor(k_base + off * KV_CHUNK + in), idesc_bf16(BN), i > 0 ? 1u : 0u);
+                if (elected()) {
+                    for (int i = 0; i < ks + rs; ++i) {
+                        const int step = i < ks ? i : kch * 4 + (i - ks);
+                        const uint32_t off = uint32_t(step / 4), in = uint32_t((step % 4) * 32);
+                        umma_ss(tmem + kColS, desc_kmajor(q_base + off * Q_CHUNK + in), desc_kmajor(k_base + off * KV_CHUNK + in), idesc_bf16(BN), i > 0 ? 1u : 0u);
+                    }
+                    umma_commit(&s_full);
                 }
-                umma_commit(&s_full);
+                __syncwarp();
             };
-            if (ok && mbar_wait(&kv_full[0], 0, &s_err)) { fence_after(); issue_s(0); }
+            if (ok && all_lanes(mbar_wait(&kv_full[0], 0, &s_err))) { fence_after(); issue_s(0); }
             else ok = false;
             const uint32_t id_v = idesc_bf16(vch * 64, true);
             for (int j = 0; j < nblk && ok; ++j) {
                 if (j + 1 < nblk) {
-                    if (!mbar_wait(&kv_full[(j + 1) % KVS], ((j + 1) / KVS) & 1, &s_err) || !mbar_wait(&s_free, j & 1, &s_err)) { ok = false; break; }
+                    if (!all_lanes(mbar_wait(&kv_full[(j + 1) % KVS], ((j + 1) / KVS) & 1, &s_err) && mbar_wait(&s_free, j & 1, &s_err))) { ok = false; break; }
                     fence_after();
                     issue_s(j + 1);
                 }
-                if (!mbar_wait(&p_full[j & 1], (j >> 1) & 1, &s_err)) { ok = false; break; }
+                if (!all_lanes(mbar_wait(&p_full[j & 1], (j >> 1) & 1, &s_err))) { ok = false; break; }
                 fence_after();
                 const uint32_t v_base = smem_u32(sKV + size_t(j % KVS) * stage_bytes) + qch * KV_CHUNK;
+                if (elected()) {
 #pragma unroll
-                for (int k16 = 0; k16 < BN / 16; ++k16)
-                    umma_ts(tmem + kColO, tmem + kColP + uint32_t((j & 1) * 32 + k16 * 8), desc_mnmajor(v_base + k16 * 2048, KV_CHUNK), id_v, (j > 0 || k16 > 0) ? 1u : 0u);
-                umma_commit(&pv_done[j & 1]);
-                umma_commit(&kv_empty[j % KVS]);
+                    for (int k16 = 0; k16 < BN / 16; ++k16)
+                        umma_ts(tmem + kColO, tmem + kColP + uint32_t((j & 1) * 32 + k16 * 8), desc_mnmajor(v_base + k16 * 2048, KV_CHUNK), id_v, (j > 0 || k16 > 0) ? 1u : 0u);
+                    umma_commit(&pv_done[j & 1]);
+                    umma_commit(&kv_empty[j % KVS]);
+                }
+                __syncwarp();
             }
             if (!ok) atomicExch(&s_err, 1);
         }

@@ -26,6 +26,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "tc5.cuh"
 
 namespace forge {
 
@@ -204,22 +205,25 @@ __global__ void __launch_bounds__(kThreads) attn_prefill_tc5_kernel(const __grid
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer: S of the next tile as soon as the score buffer has been read, then P V of this one
-        if (lane == 0) {
-            bool ok = mbar_wait(&q_full, 0, &s_err);
+        {   // the whole warp runs the loop, one elected lane issues
+            bool ok = tc5::all_lanes(mbar_wait(&q_full, 0, &s_err));
             const uint32_t q_base = smem_u32(sQ);
             auto issue_s = [&](int j) {   // S = Q K_j^T
                 const uint32_t k_base = smem_u32(sKV + size_t(j % KVS) * STAGE);
+                if (tc5::elected()) {
 #pragma unroll
-                for (int pass = 0; pass < NP; ++pass)
+                    for (int pass = 0; pass < NP; ++pass)
 #pragma unroll
-                    for (int k16 = 0; k16 < HD / 16; ++k16) {
-                        const uint32_t off = uint32_t(k16 / 4), in = uint32_t((k16 % 4) * 32);
-                        umma_ss(tmem + kColS, desc_kmajor(q_base + (pass * NCH + off) * Q_CHUNK + in), desc_kmajor(k_base + off * KV_CHUNK + in),
-                                Idesc<BN, false>::value, (pass > 0 || k16 > 0) ? 1u : 0u);
-                    }
-                umma_commit(&s_full);
+                        for (int k16 = 0; k16 < HD / 16; ++k16) {
+                            const uint32_t off = uint32_t(k16 / 4), in = uint32_t((k16 % 4) * 32);
+                            umma_ss(tmem + kColS, desc_kmajor(q_base + (pass * NCH + off) * Q_CHUNK + in), desc_kmajor(k_base + off * KV_CHUNK + in),
+                                    Idesc<BN, false>::value, (pass > 0 || k16 > 0) ? 1u : 0u);
+                        }
+                    umma_commit(&s_full);
+                }
+                __syncwarp();
             };
-            if (ok && mbar_wait(&kv_full[0], 0, &s_err)) {
+            if (ok && tc5::all_lanes(mbar_wait(&kv_full[0], 0, &s_err))) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 issue_s(0);
             } else {
@@ -227,22 +231,25 @@ __global__ void __launch_bounds__(kThreads) attn_prefill_tc5_kernel(const __grid
             }
             for (int j = 0; j < nblk && ok; ++j) {
                 if (j + 1 < nblk) {
-                    if (!mbar_wait(&kv_full[(j + 1) % KVS], ((j + 1) / KVS) & 1, &s_err) || !mbar_wait(&s_free, j & 1, &s_err)) { ok = false; break; }
+                    if (!tc5::all_lanes(mbar_wait(&kv_full[(j + 1) % KVS], ((j + 1) / KVS) & 1, &s_err) && mbar_wait(&s_free, j & 1, &s_err))) { ok = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     issue_s(j + 1);
                 }
-                if (!mbar_wait(&p_full[j & 1], (j >> 1) & 1, &s_err)) { ok = false; break; }
+                if (!tc5::all_lanes(mbar_wait(&p_full[j & 1], (j >> 1) & 1, &s_err))) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t v_base = smem_u32(sKV + size_t(j % KVS) * STAGE) + NCH * KV_CHUNK;
                 const uint32_t p_base = tmem + kColP + uint32_t((j & 1) * 64);
+                if (tc5::elected()) {
 #pragma unroll
-                for (int pass = 0; pass < NP; ++pass)
+                    for (int pass = 0; pass < NP; ++pass)
 #pragma unroll
-                    for (int k16 = 0; k16 < BN / 16; ++k16)
-                        umma_ts(tmem + kColO, p_base + uint32_t(pass * 32 + k16 * 8), desc_mnmajor(v_base + k16 * 2048, KV_CHUNK),
-                                Idesc<HD, true>::value, (j > 0 || pass > 0 || k16 > 0) ? 1u : 0u);
-                umma_commit(&pv_done[j & 1]);
-                umma_commit(&kv_empty[j % KVS]);
+                        for (int k16 = 0; k16 < BN / 16; ++k16)
+                            umma_ts(tmem + kColO, p_base + uint32_t(pass * 32 + k16 * 8), desc_mnmajor(v_base + k16 * 2048, KV_CHUNK),
+                                    Idesc<HD, true>::value, (j > 0 || pass > 0 || k16 > 0) ? 1u : 0u);
+                    umma_commit(&pv_done[j & 1]);
+                    umma_commit(&kv_empty[j % KVS]);
+                }
+                __syncwarp();
             }
             if (!ok) atomicExch(&s_err, 1);
         }

@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(kThreads<NT>, NT <= 16 ? 2 : 1) gemm_dense_ker
             cluster_sync();
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {   // the whole warp runs the loop, one elected lane issues
             int s = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -357,20 +357,23 @@ __global__ void __launch_bounds__(kThreads<NT>, NT <= 16 ? 2 : 1) gemm_dense_ker
             if constexpr (MODE != PLAIN) { pdl_wait(); groups = *p.groups.n; }
             for (Work<MODE> w(p, u0, u1, groups); ok && w.next(); ++seg) {
                 const int n = w.n, buf = seg & 1;
-                if (seg >= 2 && !mbar_wait(&acc_empty[buf], ((seg >> 1) - 1) & 1, &s_err)) { ok = false; break; }
+                if (seg >= 2 && !all_lanes(mbar_wait(&acc_empty[buf], ((seg >> 1) - 1) & 1, &s_err))) { ok = false; break; }
                 fence_after();
                 for (int k = 0; k < n; ++k) {
-                    if (!mbar_wait(&full[s], phase, &s_err)) { ok = false; break; }
+                    if (!all_lanes(mbar_wait(&full[s], phase, &s_err))) { ok = false; break; }
                     fence_after();
                     const uint32_t base = smem_u32(ring + size_t(s) * STAGE);
+                    if (elected()) {
 #pragma unroll
-                    for (int k16 = 0; k16 < BK / 16; ++k16)
-                        umma_ss(tmem + uint32_t(buf * NT), desc_kmajor(base + k16 * 32), desc_kmajor(base + 16384 + k16 * 32), idesc_bf16(NT),
-                                (k > 0 || k16 > 0) ? 1u : 0u);
-                    umma_commit(&empty[s]);
+                        for (int k16 = 0; k16 < BK / 16; ++k16)
+                            umma_ss(tmem + uint32_t(buf * NT), desc_kmajor(base + k16 * 32), desc_kmajor(base + 16384 + k16 * 32), idesc_bf16(NT),
+                                    (k > 0 || k16 > 0) ? 1u : 0u);
+                        umma_commit(&empty[s]);
+                        if (k == n - 1) umma_commit(&acc_full[buf]);
+                    }
+                    __syncwarp();
                     if (++s == STAGES) { s = 0; phase ^= 1; }
                 }
-                if (ok) umma_commit(&acc_full[buf]);
             }
             if (!ok) atomicExch(&s_err, 1);
         }

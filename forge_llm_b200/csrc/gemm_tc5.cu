@@ -28,6 +28,7 @@
 #include <cstring>
 
 #include "common.cuh"
+#include "tc5.cuh"
 
 namespace forge {
 
@@ -226,6 +227,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
                 tma_load_2d(dst, &map_hi, (kt_begin + kt) * BK, m0, &full_x[s]);
                 if (SPLIT) tma_load_2d(dst + X_TILE, &map_lo, (kt_begin + kt) * BK, m0, &full_x[s]);
             }
+            __syncwarp();
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer: D[weight row][token] += W(TMEM) * X(smem)^T
@@ -519,18 +521,19 @@ __global__ void __launch_bounds__(kSmallThreads, 1) gemm_small_kernel(const __gr
             }
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer: per group one meeting with its three partners, then 4 G products and three commits
-        if (lane == 0) {
-            for (int gi = 0; gi < ng; ++gi) {
-                const int sx = gi % XS, sw = gi % WG, ds = gi & 1;
-                if (!mbar_wait3(&full_x[sx], (gi / XS) & 1, &full_w[sw], (gi / WG) & 1, gi >= 2 ? &d_free[ds] : nullptr, ((gi >> 1) - 1) & 1, &s_err)) {
-                    atomicExch(&s_err, 1);
-                    break;
-                }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint64_t xd = umma_desc(smem_u32(sX + size_t(sx) * X_STAGE));
-                const uint32_t w_base = tmem + kWBase + uint32_t(sw * G * W_COLS);
-                const uint32_t d_base = tmem + uint32_t(ds * BG * NC);
+        // ---------------- MMA issuer: per group one meeting with its three partners, then 4 G products and three commits.  The whole warp runs the
+        // loop and one elected lane issues: addresses stay in uniform registers (a loop of one lane took about 80 clocks per instruction, this one 50)
+        for (int gi = 0; gi < ng; ++gi) {
+            const int sx = gi % XS, sw = gi % WG, ds = gi & 1;
+            if (!tc5::all_lanes(mbar_wait3(&full_x[sx], (gi / XS) & 1, &full_w[sw], (gi / WG) & 1, gi >= 2 ? &d_free[ds] : nullptr, ((gi >> 1) - 1) & 1, &s_err))) {
+                atomicExch(&s_err, 1);
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint64_t xd = umma_desc(smem_u32(sX + size_t(sx) * X_STAGE));
+            const uint32_t w_base = tmem + kWBase + uint32_t(sw * G * W_COLS);
+            const uint32_t d_base = tmem + uint32_t(ds * BG * NC);
+            if (tc5::elected()) {
 #pragma unroll
                 for (int g = 0; g < G; ++g)
 #pragma unroll
@@ -570,10 +573,6 @@ __global__ void __launch_bounds__(kSmallThreads, 1) gemm_small_kernel(const __gr
                     const uint4 v = *reinterpret_cast<const uint4*>(stage + box * 16384 + r * 128 + ((uint32_t(piece) ^ sw7) << 4));
                     cur[4 * i] = v.x; cur[4 * i + 1] = v.y; cur[4 * i + 2] = v.z; cur[4 * i + 3] = v.w;
                 }
-                if (qi == kSuper - 1 || kt == ng * G - 1) {   // the stage's bytes are in registers
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&empty_q[sq]);
-                }
                 uint32_t w16[16];
                 raw_block<QUANT>(cur, w16);
                 if (g == 0) {   // first K step of a group: its stage must have been read by the products that used it last
@@ -582,6 +581,10 @@ __global__ void __launch_bounds__(kSmallThreads, 1) gemm_small_kernel(const __gr
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 }
                 tmem_st16(lane_base + uint32_t((sw * G + g) * W_COLS), w16);
+                if (qi == kSuper - 1 || kt == ng * G - 1) {   // what the stage held has been used
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&empty_q[sq]);
+                }
                 if (g == G - 1) {   // the group is complete
                     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

@@ -70,6 +70,15 @@ __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64
     asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
                  ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(id), "r"(accumulate) : "memory");
 }
+// One lane of a converged warp, always the same one.  A warp that runs its loop as a whole and lets this lane issue keeps descriptors and addresses in uniform
+// registers: a product or commit then costs about 50 clocks to issue, in a loop of one lane about 80.
+__device__ __forceinline__ bool elected() {
+    uint32_t e;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(e));
+    return e != 0;
+}
+// such a warp's waits: all lanes go on, or none does
+__device__ __forceinline__ bool all_lanes(bool x) { return __all_sync(0xffffffffu, x); }
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
