@@ -1,4 +1,4 @@
-"""Products on CTA pairs and the decode attention at the sizes where their tiles, slices and splits begin and end.
+"""Products of prompts and the decode attention at the sizes where their tiles, slices and splits begin and end.
 
 Tolerances: the products carry both operands to 22 bits; their error is the tensor core's rounding toward zero, which grows with K and
 stays below 3e-5 at K = 8192 (the bound of the batched products' own test, 6e-5, holds with room).  The decode attention carries queries and
@@ -14,9 +14,9 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("quant", [8, 4])
 @pytest.mark.parametrize("m,K,N", [(33, 64, 2), (64, 256, 256), (65, 320, 257), (128, 64, 130), (129, 192, 300), (191, 576, 254), (193, 128, 512), (256, 1024, 20), (257, 448, 131),
                                    (700, 2048, 18992)])
-def test_pair_product_edges(oracle, quant, m, K, N):
-    """Token tiles of 64 .. 256, row tiles of 256 in halves, K of one step, of part of a stage, of several stages, outputs with and without bulk
-    stores (N a multiple of 4 or not, a buffer that does not begin on 16 bytes), several tiles per CTA pair."""
+def test_prompt_product_edges(oracle, quant, m, K, N):
+    """Token tiles, row tiles, K of one step, of part of a stage, of several stages, outputs with and without
+    aligned rows (N a multiple of 4 or not, a buffer that does not begin on 16 bytes), several rounds of tiles."""
     import ctypes as C
     import torch
     from forge_llm_b200 import synth
