@@ -227,7 +227,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
                 tma_load_2d(dst, &map_hi, (kt_begin + kt) * BK, m0, &full_x[s]);
                 if (SPLIT) tma_load_2d(dst + X_TILE, &map_lo, (kt_begin + kt) * BK, m0, &full_x[s]);
             }
-            __syncwarp();
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer: D[weight row][token] += W(TMEM) * X(smem)^T
@@ -544,6 +543,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) gemm_small_kernel(const __gr
                 umma_commit(&empty_x[sx]);
                 umma_commit(&empty_w[sw]);
             }
+            __syncwarp();
         }
     } else if (warp < 10) {
         // ---------------- dequantise (warps 2..9): integer weights as fp16 into tensor memory, lane = weight row
