@@ -12,12 +12,10 @@
 // head_dim 64 whatever the group; with scores and sums formed by fused multiply-adds (four heads per pass over the page) one page took 1.7 us.
 // The splits of a (sequence, KV head) are a cluster and merge through distributed shared memory; beyond eight splits (contexts past 128 pages) the
 // last CTA to finish merges partials from global memory (atomic ticket).  Every wait is bounded.
-#include <cuda.h>
-
 #include <algorithm>
 #include <mutex>
 
-#include "common.cuh"
+#include "attn_decode.cuh"
 #include "mma.cuh"
 #include "tc5.cuh"
 
@@ -25,75 +23,15 @@ namespace forge {
 
 namespace {
 
+using namespace decode;
 using tc5::cluster_addr;
 using tc5::cluster_sync;
 
-constexpr int kThreads = 128;     // consumer threads (four warps); warp 4 is the producer
-constexpr int kBlock = kThreads + 32;
-constexpr int kStages = 4;        // most pages (K and V) in flight per CTA
-constexpr int kMaxGroup = 16;     // query heads per KV head
-constexpr int kHeads = 8;         // of them in one pass over the keys
-constexpr int kMaxSplits = 32;    // context splits per KV head
-constexpr int kClusterSplits = 8; // of them in a cluster
-constexpr uint32_t kSpin = 1u << 22;
+constexpr int kHeads = 8;         // query heads of a KV head in one pass over the keys
+constexpr int kClusterSplits = 8; // context splits in a cluster
 constexpr float kLog2e = 1.4426950408889634f;
 
-struct DecParams {
-    AttnDecodeArgs a;
-    float scale;  // of the scores, times log2 e
-    int stages;   // ring depth of this launch (<= kStages)
-};
-
 __device__ __forceinline__ float exp2_rel(float x, float m) { return x == -INFINITY ? 0.f : exp2f(x - m); }   // 0 for an empty part, never NaN
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-    const uint32_t addr = smem_u32(bar);
-    for (uint32_t i = 0; i < kSpin; ++i) {
-        uint32_t done;
-        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
-                     : "=r"(done) : "r"(addr), "r"(parity) : "memory");
-        if (done) return true;
-    }
-    return false;
-}
-// 64 dimensions of one page of one KV head: box {64, 1, 64 rows} at {dimension, kv head, row}
-__device__ __forceinline__ void tma_page(void* dst, const CUtensorMap* map, int dim, int kvh, int row, uint64_t* bar) {
-    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-                 ::"r"(smem_u32(dst)), "l"(map), "r"(dim), "r"(kvh), "r"(row), "r"(smem_u32(bar)) : "memory");
-}
-// the result in the form the caller asked for: f32, or fp16 hi (+ lo)
-__device__ __forceinline__ void store_out(const AttnDecodeArgs& a, size_t i, float x) {
-    if (a.out16) {
-        const __half h = __float2half_rn(x);
-        a.out16[i] = h;
-        if (a.out16_lo) a.out16_lo[i] = __float2half_rn(x - __half2float(h));
-    } else {
-        a.out[i] = x;
-    }
-}
-__device__ __forceinline__ void store_out2(const AttnDecodeArgs& a, size_t i, float2 x) {
-    if (a.out16) {
-        const __half2 h = __floats2half2_rn(x.x, x.y);
-        *reinterpret_cast<__half2*>(a.out16 + i) = h;
-        if (a.out16_lo) {
-            const float2 hf = __half22float2(h);
-            *reinterpret_cast<__half2*>(a.out16_lo + i) = __floats2half2_rn(x.x - hf.x, x.y - hf.y);
-        }
-    } else {
-        *reinterpret_cast<float2*>(a.out + i) = x;
-    }
-}
-__device__ __forceinline__ void csync() { asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory"); }
 
 __device__ __forceinline__ void mma16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -400,6 +338,7 @@ int32_t launch_decode(const CUtensorMap& mk, const CUtensorMap& mv, const DecPar
 }
 
 int32_t attn_decode(const AttnDecodeArgs& a, cudaStream_t st) {
+    if (a.f32) return attn_decode_f32(a, st);
     if (a.nq % a.nkv) { set_error("attention: num_heads %d not a multiple of num_kv_heads %d", a.nq, a.nkv); return FORGE_ERR_SHAPE; }
     if (a.splits < 1 || (a.splits > kClusterSplits && (!a.ws || !a.counters))) { set_error("attention: split workspace missing"); return FORGE_ERR_INVALID_ARG; }
     if (a.nq / a.nkv > kMaxGroup) { set_error("attention: at most %d query heads per KV head", kMaxGroup); return FORGE_ERR_SHAPE; }

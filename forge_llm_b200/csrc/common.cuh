@@ -269,15 +269,22 @@ struct AttnDecodeArgs {
     // out16 != null: the result is stored as fp16 hi (+ lo) rows [batch][nq*hd] (the operand of a tensor-core product)
     // instead of f32 `out`
     __half* out16 = nullptr; __half* out16_lo = nullptr;
+    // scores and sums by f32 multiply-adds in a fixed order (attn_decode_f32.cu): for results that are rounded to 8 bits next.  Splits, workspace and
+    // tensor maps are then those of the _f32 functions
+    bool f32 = false;
 };
 // context splits for `groups` = batch * kv_heads independent (sequence, KV head) pairs over `pages` pages.  Up to eight need no
 // workspace (attn_decode_ws_floats is 0): a.ws and a.counters may then be null
 int attn_decode_splits(int pages, int groups, int sms, int hd, int heads_per_group);
 size_t attn_decode_ws_floats(int batch, int nq, int hd, int splits);
+int attn_decode_f32_splits(int pages, int groups, int sms, int hd, int heads_per_group);
+size_t attn_decode_f32_ws_floats(int batch, int nq, int hd, int splits);
 // Tiled tensor map over an fp16 K or V pool of `rows` rows of kv_heads * head_dim values: dimensions {head_dim, kv_heads,
-// rows}, box {64, 1, 64} = 64 dimensions of one page of one KV head, SWIZZLE_128B (`out`: a CUtensorMap in host memory)
-int32_t make_kv_map(void* out, const __half* pool, int head_dim, int kv_heads, size_t rows);
+// rows}, box {64, 1, 64} = 64 dimensions of one page of one KV head, SWIZZLE_128B (`out`: a CUtensorMap in host memory).  f32: for attn_decode_f32,
+// box {head_dim, 1, 64}, rows as they lie in memory
+int32_t make_kv_map(void* out, const __half* pool, int head_dim, int kv_heads, size_t rows, bool f32 = false);
 int32_t attn_decode(const AttnDecodeArgs& a, cudaStream_t st);
+int32_t attn_decode_f32(const AttnDecodeArgs& a, cudaStream_t st);
 
 struct AttnPrefillArgs {
     __half* out16; __half* out16_lo; float* out32;  // out16 (+ optional lo part) or out32: [m][nq*hd]

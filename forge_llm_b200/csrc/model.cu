@@ -330,7 +330,7 @@ struct PrefillToken { int seq; const uint32_t* tok; bool head; float* trace_dst;
 constexpr int kBatchGroup = 16;
 // splits of the decode attention for the sequences of one launch; the workspace of more than eight was made for all of the cache's
 int launch_splits(const ForgeModel* m, const ForgeKV* kv, int batch) {
-    if (batch >= kv->batch) return kv->splits;
+    if (batch >= kv->batch || m->any_kquant) return kv->splits;
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device);
     const int s = attn_decode_splits(kv->pages_per_seq, batch * m->nkv, sms, m->hd, m->nq / m->nkv);
@@ -428,7 +428,7 @@ int32_t decode_launches_batched(ForgeModel* m, ForgeKV* kv, int batch, bool gree
                                 m->qk, m->kv, m->hd, st));
         AttnDecodeArgs da{m->d_attn, m->d_q, kp, vp, kv->d_page_table, kv->pages_per_seq, kv->d_seq_len, 0,
                           n, m->nq, m->nkv, m->hd, kv->max_seq, kv->attn_ws, kv->attn_counters, launch_splits(m, kv, n), c.sliding_window};
-        da.map_k = kv->k_map; da.map_v = kv->v_map; da.row_base = int(size_t(l) * kv->num_pages * FORGE_KV_PAGE); da.err = m->d_err;
+        da.map_k = kv->k_map; da.map_v = kv->v_map; da.row_base = int(size_t(l) * kv->num_pages * FORGE_KV_PAGE); da.err = m->d_err; da.f32 = m->any_kquant;
         FORGE_TRY(attn_decode(da, st));
         FORGE_TRY(batched_row_sliced(m, L.o_t, m->d_attn, m->qk, PLAIN, n, &sums, &pending, st));
         FORGE_TRY(normed_product(L.gateup_t, L.ffn_norm, m->p_gu));
@@ -467,7 +467,7 @@ int32_t decode_launches_gemm(ForgeModel* m, ForgeKV* kv, int batch, bool greedy,
                                 kv->pages_per_seq, m->qk, m->kv, m->hd, st, qks, qstride));
         AttnDecodeArgs da{m->d_attn, m->d_q, kp, vp, kv->d_page_table, kv->pages_per_seq, kv->d_seq_len, 0,
                           n, m->nq, m->nkv, m->hd, kv->max_seq, kv->attn_ws, kv->attn_counters, launch_splits(m, kv, n), c.sliding_window};
-        da.map_k = kv->k_map; da.map_v = kv->v_map; da.row_base = int(size_t(l) * kv->num_pages * FORGE_KV_PAGE); da.err = m->d_err;
+        da.map_k = kv->k_map; da.map_v = kv->v_map; da.row_base = int(size_t(l) * kv->num_pages * FORGE_KV_PAGE); da.err = m->d_err; da.f32 = m->any_kquant;
         da.out16 = m->p_attn16; da.out16_lo = alo;   // straight into the o-projection's operand form
         FORGE_TRY(attn_decode(da, st));
         FORGE_TRY(row_sliced_gemm_norm(m, L.o, m->p_attn16, alo, n, L.ffn_norm, nlo, st));
@@ -543,7 +543,7 @@ int32_t decode_launches(ForgeModel* m, ForgeKV* kv, int batch, bool greedy, bool
         }
         AttnDecodeArgs da{m->d_attn, m->d_q, kp, vp, page_table, kv->pages_per_seq, seq_len, 0,
                           batch, m->nq, m->nkv, m->hd, kv->max_seq, kv->attn_ws, kv->attn_counters, launch_splits(m, kv, batch), c.sliding_window};
-        da.map_k = kv->k_map; da.map_v = kv->v_map; da.row_base = int(size_t(l) * kv->num_pages * FORGE_KV_PAGE); da.err = m->d_err;
+        da.map_k = kv->k_map; da.map_v = kv->v_map; da.row_base = int(size_t(l) * kv->num_pages * FORGE_KV_PAGE); da.err = m->d_err; da.f32 = m->any_kquant;
         FORGE_TRY(attn_decode(da, st));
         GemvArgs o;
         o.x = m->d_attn; o.out = hid[cur]; o.resid = hid[cur]; o.batch = batch;
@@ -920,8 +920,8 @@ int32_t forge_kv_create_pool(ForgeModel* m, int32_t pool_tokens, int32_t max_seq
     static_assert(sizeof(kv->k_map) >= 128, "CUtensorMap is 128 bytes");
     {
         const size_t rows = size_t(kv->num_pages) * FORGE_KV_PAGE * m->cfg.num_layers;
-        int32_t rc = make_kv_map(kv->k_map, kv->k_pool, m->hd, m->nkv, rows);
-        if (rc == FORGE_OK) rc = make_kv_map(kv->v_map, kv->v_pool, m->hd, m->nkv, rows);
+        int32_t rc = make_kv_map(kv->k_map, kv->k_pool, m->hd, m->nkv, rows, m->any_kquant);
+        if (rc == FORGE_OK) rc = make_kv_map(kv->v_map, kv->v_pool, m->hd, m->nkv, rows, m->any_kquant);
         if (rc != FORGE_OK) return fail(rc);
     }
     cudaMemsetAsync(kv->k_pool, 0, pool * sizeof(__half), m->stream);
@@ -940,8 +940,8 @@ int32_t forge_kv_create_pool(ForgeModel* m, int32_t pool_tokens, int32_t max_seq
     if (!m->stack) {
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device);
-    kv->splits = attn_decode_splits(kv->pages_per_seq, batch * m->nkv, sms, m->hd, m->nq / m->nkv);
-    if (cudaMalloc(&kv->attn_ws, sizeof(float) * attn_decode_ws_floats(batch, m->nq, m->hd, kv->splits)) != cudaSuccess ||
+    kv->splits = (m->any_kquant ? attn_decode_f32_splits : attn_decode_splits)(kv->pages_per_seq, batch * m->nkv, sms, m->hd, m->nq / m->nkv);
+    if (cudaMalloc(&kv->attn_ws, sizeof(float) * (m->any_kquant ? attn_decode_f32_ws_floats : attn_decode_ws_floats)(batch, m->nq, m->hd, kv->splits)) != cudaSuccess ||
         cudaMalloc(&kv->attn_counters, sizeof(int) * batch * m->nkv) != cudaSuccess) { set_error("attention workspace allocation failed"); return fail(FORGE_ERR_CUDA); }
     cudaMemsetAsync(kv->attn_counters, 0, sizeof(int) * batch * m->nkv, m->stream);
     }
