@@ -60,9 +60,9 @@ __global__ void __launch_bounds__(kBlock, HD == 64 ? 3 : 2) attn_decode_kernel(c
     constexpr int KS = HD / 16, NV = HD / 8;
     extern __shared__ __align__(1024) unsigned char ring_raw[];   // [stages][K page | V page], then [warp][head][HD] sums
     unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(ring_raw) + 1023) & ~uintptr_t(1023));
-    float* s_acc = reinterpret_cast<float*>(ring + size_t(p.stages) * 2 * PAGE_BYTES);   // in the end [head][HD] of the CTA
+    float* s_acc = reinterpret_cast<float*>(ring + size_t(p.stages) * 2 * PAGE_BYTES);
     __shared__ uint64_t full_bar[kStages], empty_bar[kStages];
-    __shared__ float s_ml[4][kHeads][2], s_cml[kHeads][2];
+    __shared__ float s_ml[4][kHeads][2], s_cml[kMaxGroup][2];
     __shared__ float s_fw[kMaxSplits][kMaxGroup];         // global merge: weight of split s for query head g
     __shared__ int s_last;
     const AttnDecodeArgs& a = p.a;
@@ -70,6 +70,7 @@ __global__ void __launch_bounds__(kBlock, HD == 64 ? 3 : 2) attn_decode_kernel(c
     const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lr = lane >> 2, lc = (lane & 3) * 2;
     const int G = a.nq / a.nkv, kvd = a.nkv * HD;
+    float* s_sum = G > kHeads ? s_acc + 4 * kHeads * HD : s_acc;   // [head][HD] sums of the CTA (of one pass: over warp 0's own values)
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], kThreads / 32); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -228,42 +229,42 @@ __global__ void __launch_bounds__(kBlock, HD == 64 ? 3 : 2) attn_decode_kernel(c
             if (a.splits == 1) {
                 store_out(a, (size_t(b) * a.nq + kvh * G + g0) * HD + idx, A * (1.0f / L));
             } else if (CL) {
-                s_acc[idx] = A;   // over warp 0's own value
-                if (idx % HD == 0) { s_cml[g][0] = M; s_cml[g][1] = L; }
+                s_sum[g0 * HD + idx] = A;
+                if (idx % HD == 0) { s_cml[g0 + g][0] = M; s_cml[g0 + g][1] = L; }
             } else {
                 float* w = a.ws + ((size_t(b) * a.nq + kvh * G + g0 + g) * a.splits + split) * (HD + 2);
                 w[2 + idx % HD] = A;
                 if (idx % HD == 0) { w[0] = M; w[1] = L; }
             }
         }
-        if (CL && a.splits > 1) {
-            // ---- the CTAs' parts become the result, each CTA finishing a share of it
-            cluster_sync();
-            const int items = gc * HD, share = (items + a.splits - 1) / a.splits;
-            for (int idx = split * share + threadIdx.x; idx < min(items, (split + 1) * share); idx += kThreads) {
-                const int g = idx / HD;
-                float pm[kClusterSplits], pl[kClusterSplits], px[kClusterSplits], M = -INFINITY, A = 0.f, L = 0.f;
+        csync();
+    }
+    if (CL && a.splits > 1) {
+        // ---- the CTAs' parts become the result, each CTA finishing a share of it.  Only here, behind the last pass: until then the producer lane may be
+        // waiting for ring space, and a cluster waits for every thread that has not left
+        cluster_sync();
+        const int items = G * HD, share = (items + a.splits - 1) / a.splits;
+        for (int idx = split * share + threadIdx.x; idx < min(items, (split + 1) * share); idx += kThreads) {
+            const int g = idx / HD;
+            float pm[kClusterSplits], pl[kClusterSplits], px[kClusterSplits], M = -INFINITY, A = 0.f, L = 0.f;
 #pragma unroll
-                for (int s = 0; s < kClusterSplits; ++s) {
-                    const bool on = s < a.splits;
-                    pm[s] = on ? remote_f32(cluster_addr(&s_cml[g][0], s)) : -INFINITY;
-                    pl[s] = on ? remote_f32(cluster_addr(&s_cml[g][1], s)) : 0.f;
-                    px[s] = on ? remote_f32(cluster_addr(s_acc + idx, s)) : 0.f;
-                }
-#pragma unroll
-                for (int s = 0; s < kClusterSplits; ++s) M = fmaxf(M, pm[s]);
-#pragma unroll
-                for (int s = 0; s < kClusterSplits; ++s) {
-                    const float f = exp2_rel(pm[s], M);
-                    A += px[s] * f;
-                    L += pl[s] * f;
-                }
-                store_out(a, (size_t(b) * a.nq + kvh * G + g0) * HD + idx, A * (1.0f / L));
+            for (int s = 0; s < kClusterSplits; ++s) {
+                const bool on = s < a.splits;
+                pm[s] = on ? remote_f32(cluster_addr(&s_cml[g][0], s)) : -INFINITY;
+                pl[s] = on ? remote_f32(cluster_addr(&s_cml[g][1], s)) : 0.f;
+                px[s] = on ? remote_f32(cluster_addr(s_sum + idx, s)) : 0.f;
             }
-            cluster_sync();   // nobody leaves, or starts the next heads, while its sums are read
-        } else {
-            csync();
+#pragma unroll
+            for (int s = 0; s < kClusterSplits; ++s) M = fmaxf(M, pm[s]);
+#pragma unroll
+            for (int s = 0; s < kClusterSplits; ++s) {
+                const float f = exp2_rel(pm[s], M);
+                A += px[s] * f;
+                L += pl[s] * f;
+            }
+            store_out(a, (size_t(b) * a.nq + size_t(kvh) * G) * HD + idx, A * (1.0f / L));
         }
+        cluster_sync();   // nobody leaves while its sums are read
     }
     if (CL || a.splits == 1) return;
 
@@ -328,8 +329,8 @@ size_t attn_decode_ws_floats(int batch, int nq, int hd, int splits) { return spl
 
 template <int HD, bool SW>
 int32_t launch_decode(const CUtensorMap& mk, const CUtensorMap& mv, const DecParams& p, dim3 grid, cudaStream_t st) {
-    constexpr int kPage = (HD + 63) / 64 * FORGE_KV_PAGE * 128, kSums = 4 * kHeads * HD * 4;
-    const size_t smem = size_t(p.stages) * 2 * kPage + kSums + 1024;
+    constexpr int kPage = (HD + 63) / 64 * FORGE_KV_PAGE * 128, kSums = (4 * kHeads + kMaxGroup) * HD * 4;
+    const size_t smem = size_t(p.stages) * 2 * kPage + (p.a.nq > kHeads * p.a.nkv ? kSums : 4 * kHeads * HD * 4) + 1024;
     auto kern = p.a.splits <= kClusterSplits ? attn_decode_kernel<HD, SW, true> : attn_decode_kernel<HD, SW, false>;
     FORGE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kStages * 2 * kPage + kSums + 1024));
     FORGE_CUDA(launch_pdl_cluster(kern, grid, dim3(kBlock), p.a.splits <= kClusterSplits ? p.a.splits : 1, smem, st, mk, mv, p));

@@ -29,3 +29,71 @@ def test_kquant_steps_keep_their_logits():
     then moves a whole step of that rounding (6e-3 of a step's logits here).  The stored logits are those of attention by f32 multiply-adds in a
     fixed order; 1e-6 leaves room for f32 rounding and for no such step."""
     assert rel_l2(kquant_steps(), np.load(GOLDEN)["logits"]) < 1e-6
+
+
+def attend(q, k, v, seq, window=0, fn=None):
+    """The operator's result for float32 queries [heads][hd] over fp16 rows [seq][kv heads][hd], everything on the GPU."""
+    import torch
+    from forge_llm_b200._lib import check, lib
+    (nq, hd), nkv = q.shape, k.shape[1]
+    out = torch.full((nq, hd), 7.0, device="cuda")
+    p = [x.data_ptr() for x in (out, q, k, v)]
+    if window:
+        check(lib.forge_attention_sliding(*p, seq, window, nq, nkv, hd, None))
+    else:
+        check((fn or lib.forge_attention_flash)(*p, seq, nq, nkv, hd, None))
+    torch.cuda.synchronize()
+    return out
+
+
+def attend64(q, k, v, seq, window=0):
+    """The same in 64 bits."""
+    import torch
+    (nq, hd), nkv = q.shape, k.shape[1]
+    lo = max(0, seq - window) if window else 0
+    s = torch.einsum("ngd,tnd->ngt", q.double().view(nkv, nq // nkv, hd), k[lo:seq].double()) / hd ** 0.5
+    p = torch.exp(s - s.amax(-1, keepdim=True))
+    return (torch.einsum("ngt,tnd->ngd", p, v[lo:seq].double()) / p.sum(-1, keepdim=True)).reshape(nq, hd)
+
+
+def inputs(hd, nq, nkv, seq, q_scale=1.0, k_scale=0.5):
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(hd + 7 * nq + 31 * nkv + seq)
+    q = q_scale * torch.randn(nq, hd, generator=g, device="cuda")
+    k, v = torch.randn(2, seq, nkv, hd, generator=g, device="cuda")
+    return q, (k_scale * k).half(), v.half()
+
+
+def error(got, want):
+    return ((got.double() - want).norm() / want.norm()).item()
+
+
+@pytest.mark.parametrize("hd,nq,nkv", [(64, 9, 1), (64, 32, 2), (96, 12, 1), (128, 16, 1), (128, 24, 2)])
+@pytest.mark.parametrize("seq,window", [(1100, 0), (2100, 0), (4096, 0), (8192, 0), (8191, 3000), (8300, 0), (8300, 5000)])
+def test_two_passes_over_more_pages_than_the_ring_holds(hd, nq, nkv, seq, window):
+    """Nine to sixteen query heads per KV head take two passes over a CTA's pages; here the pages of the first pass fill the ring, so that the copies
+    of the second can only begin as pages are read, and the CTAs of a cluster meet behind both."""
+    from forge_llm_b200._lib import lib
+    q, k, v = inputs(hd, nq, nkv, seq)
+    want = attend64(q, k, v, seq, window)
+    assert error(attend(q, k, v, seq, window), want) < 3e-6
+    if not window:
+        assert error(attend(q, k, v, seq, fn=lib.forge_attention_flash_static), want) < 3e-6
+
+
+@pytest.mark.parametrize("hd,nq,nkv", [(64, 16, 1), (128, 12, 1)])
+def test_steps_of_models_with_many_heads_per_kv_head(hd, nq, nkv):
+    """The same through a session: a step behind n tokens gives the logits of a prompt of n + 1 (the prompt's attention is another kernel)."""
+    from forge_llm_b200 import configs, runtime, synth
+    c = configs.tiny(8, hd=hd, nq=nq, nkv=nkv, layers=2)
+    gm = runtime.Model(c, synth.make_weights_bin(c))
+    toks = synth.prompt_tokens(c, 3001)
+    kv = gm.new_cache(max_seq=3100)
+    want = gm.forward_prefill(toks, kv)
+    kv.reset()
+    gm.forward_prefill(toks[:3000], kv, want_logits=False)
+    got = gm.forward(int(toks[3000]), kv)
+    assert rel_l2(got, want) < 1e-3    # the prompt's queries and weights enter its products as plain fp16
+    kv.close()
+    gm.close()
