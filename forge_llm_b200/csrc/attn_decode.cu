@@ -7,12 +7,16 @@
 // newest was written by earlier steps.
 //
 // Four consumer warps take sixteen keys of a page each, as mma.sync products: up to eight query heads of the group are rows 0..7 of the A tile as fp16 hi
-// parts and rows 8..15 as lo parts, so that one product serves both halves of the 22-bit query and a thread adds them from its own registers; the probabilities
-// enter their product with the values the same way.  Softmax state is f32.  A page costs a warp about forty tensor instructions at
-// head_dim 64 whatever the group; with scores and sums formed by fused multiply-adds (four heads per pass over the page) one page took 1.7 us.
+// parts and rows 8..15 as lo parts, so that one product serves both halves of the query and a thread adds them from its own registers; the weights
+// enter their product with the values the same way.  A power of two in front of either split keeps all bits of it in fp16's range, no
+// product is carried further than its neighbour, and f32 sums take over: against 64 bits the result is nearer than f32 multiply-adds bring it (0.9 of their
+// error for scores around 1, 0.65 around 10; 8000 keys of one weight 1.6e-7, 3.8e-7 with sums carried through the tensor core).
+// A page costs a warp about forty tensor instructions at head_dim 64 whatever the group; with scores and sums
+// formed by fused multiply-adds (four heads per pass over the page) one page took 1.7 us.
 // The splits of a (sequence, KV head) are a cluster and merge through distributed shared memory; beyond eight splits (contexts past 128 pages) the
 // last CTA to finish merges partials from global memory (atomic ticket).  Every wait is bounded.
 #include <algorithm>
+#include <cmath>
 #include <mutex>
 
 #include "attn_decode.cuh"
@@ -29,7 +33,7 @@ using tc5::cluster_sync;
 
 constexpr int kHeads = 8;         // query heads of a KV head in one pass over the keys
 constexpr int kClusterSplits = 8; // context splits in a cluster
-constexpr float kLog2e = 1.4426950408889634f;
+constexpr float kUp = 32768.f;    // of a weight in front of its product: the lo part of 2^-14 of the largest one is still a normal fp16 number
 
 __device__ __forceinline__ float exp2_rel(float x, float m) { return x == -INFINITY ? 0.f : exp2f(x - m); }   // 0 for an empty part, never NaN
 
@@ -113,24 +117,39 @@ __global__ void __launch_bounds__(kBlock, HD == 64 ? 3 : 2) attn_decode_kernel(c
 
     for (int g0 = 0; g0 < G; g0 += kHeads) {
         const int gc = min(kHeads, G - g0);
-        // A fragments of the scaled queries: row lr = hi part of head lr, row lr + 8 = lo part
+        // A fragments of the queries: row lr = hi part of head lr, row lr + 8 = lo part.  A power of two takes the head's largest value to [2^14, 2^15), so that
+        // the parts hold what they can of any size of query and none overflows; `unit` takes a score back, and to powers of two
         uint32_t qf[KS][4];
+        float unit, unit_lo;
+        {
+            float q[KS][4], big = 0.f;
 #pragma unroll
-        for (int k = 0; k < KS; ++k) {
-            float2 x = make_float2(0.f, 0.f), y = x;
-            if (lr < gc) {
-                const float* qp = a.q + (size_t(b) * a.nq + kvh * G + g0 + lr) * HD + k * 16 + lc;
-                x = *reinterpret_cast<const float2*>(qp);
-                y = *reinterpret_cast<const float2*>(qp + 8);
+            for (int k = 0; k < KS; ++k) {
+                float2 x = make_float2(0.f, 0.f), y = x;
+                if (lr < gc) {
+                    const float* qp = a.q + (size_t(b) * a.nq + kvh * G + g0 + lr) * HD + k * 16 + lc;
+                    x = *reinterpret_cast<const float2*>(qp);
+                    y = *reinterpret_cast<const float2*>(qp + 8);
+                }
+                q[k][0] = x.x; q[k][1] = x.y; q[k][2] = y.x; q[k][3] = y.y;
+                big = fmaxf(fmaxf(big, fmaxf(fabsf(x.x), fabsf(x.y))), fmaxf(fabsf(y.x), fabsf(y.y)));
             }
-            split_h2(x.x * p.scale, x.y * p.scale, qf[k][0], qf[k][1]);
-            split_h2(y.x * p.scale, y.y * p.scale, qf[k][2], qf[k][3]);
+            big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, 1));
+            big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, 2));
+            const int up = min(268 - (__float_as_int(big) >> 23), 253);   // exponent fields: 2^(up - 127) is the factor, 2^(127 - up) takes it back
+            const float f = __int_as_float(up << 23);
+            unit = __int_as_float((254 - up) << 23) * p.scale;
+            unit_lo = __int_as_float((254 - up) << 23) * p.scale_lo;
+#pragma unroll
+            for (int k = 0; k < KS; ++k) {
+                split_h2(q[k][0] * f, q[k][1] * f, qf[k][0], qf[k][1]);
+                split_h2(q[k][2] * f, q[k][3] * f, qf[k][2], qf[k][3]);
+            }
         }
-        float o[NV][4], m = -INFINITY, l = 0.f;
+        // sums relative to 2^m: of the values (times kUp), of the weights
+        float o[NV][2], m = -INFINITY, l = 0.f;
 #pragma unroll
-        for (int v = 0; v < NV; ++v)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) o[v][e] = 0.f;
+        for (int v = 0; v < NV; ++v) o[v][0] = o[v][1] = 0.f;
         for (int lp = split; lp < n_pages; lp += a.splits) {
             if (SW && (lp + 1) * FORGE_KV_PAGE <= t_first) continue;  // the whole page lies before the window
             const int t0 = lp * FORGE_KV_PAGE + warp * 16;            // the warp's sixteen keys
@@ -158,48 +177,66 @@ __global__ void __launch_bounds__(kBlock, HD == 64 ? 3 : 2) attn_decode_kernel(c
                 }
                 const uint32_t kb = smem_u32(ks), vb = kb + PAGE_BYTES;
                 const uint32_t krow = kb + uint32_t((lane & 7) + ((lane >> 4) << 3)) * 128, vrow = vb + uint32_t(lane & 15) * 128;
-                float s[2][2][4];   // [key tile][even and odd steps][fragment]
+                // Two products in a row, then sums in f32 that keep what they round away (in front of which it stands with the lo parts): the additions of eight
+                // score terms in f32 alone were half of the result's error, and a longer chain of products rounds toward zero once per step
+                float s[2][2][2] = {};   // [key tile][key][hi part, rest]
 #pragma unroll
-                for (int e = 0; e < 16; ++e) s[e >> 3][(e >> 2) & 1][e & 3] = 0.f;
+                for (int k0 = 0; k0 < KS; k0 += 2) {
+                    float d[2][4] = {};
 #pragma unroll
-                for (int k = 0; k < KS; ++k) {
-                    uint32_t f[4];
-                    const uint32_t c = uint32_t(2 * k + ((lane >> 3) & 1));   // 16-byte piece of the row
-                    ldsm4(f, krow + (c >> 3) * BOX_BYTES + (((c & 7) ^ sw) << 4));
-                    mma16(s[0][k & 1], qf[k], f[0], f[1]);
-                    mma16(s[1][k & 1], qf[k], f[2], f[3]);
+                    for (int k = k0; k < k0 + 2; ++k) {
+                        uint32_t f[4];
+                        const uint32_t c = uint32_t(2 * k + ((lane >> 3) & 1));   // 16-byte piece of the row
+                        ldsm4(f, krow + (c >> 3) * BOX_BYTES + (((c & 7) ^ sw) << 4));
+                        mma16(d[0], qf[k], f[0], f[1]);
+                        mma16(d[1], qf[k], f[2], f[3]);
+                    }
+#pragma unroll
+                    for (int t = 0; t < 2; ++t)
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            if (k0 == 0) { s[t][e][0] = d[t][e]; s[t][e][1] = d[t][e + 2]; continue; }
+                            const float x = s[t][e][0], y = d[t][e], sum = x + y, z = sum - x;
+                            s[t][e][0] = sum;
+                            s[t][e][1] += ((x - (sum - z)) + (y - z)) + d[t][e + 2];
+                        }
                 }
                 float sc[4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    const int t = j >> 1, e = j & 1, key = t0 + t * 8 + lc + e;
-                    sc[j] = (s[t][0][e] + s[t][1][e]) + (s[t][0][e + 2] + s[t][1][e + 2]);
-                    if (key >= n_ctx || (SW && key < t_first)) sc[j] = -INFINITY;
+                    const int key = t0 + (j >> 1) * 8 + lc + (j & 1);
+                    sc[j] = key < n_ctx && (!SW || key >= t_first) ? s[j >> 1][j & 1][0] : -INFINITY;
                 }
                 float mn = fmaxf(fmaxf(sc[0], sc[1]), fmaxf(sc[2], sc[3]));
                 mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 1));
                 mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 2));
-                mn = fmaxf(mn, m);
+                mn = fmaxf(mn * unit, m);
                 const float at = mn == -INFINITY ? 0.f : mn, es = exp2f(m - at);   // a tile holds a visible key, but its score may be -inf
                 float pr[4];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) pr[j] = exp2f(sc[j] - at);
+                for (int j = 0; j < 4; ++j) {
+                    const float hi = s[j >> 1][j & 1][0], rest = s[j >> 1][j & 1][1];
+                    const float x = fmaf(rest, unit, fmaf(hi, unit_lo, fmaf(hi, unit, -at)));
+                    pr[j] = sc[j] == -INFINITY ? 0.f : exp2f(x);
+                }
                 m = mn;
                 l = l * es + ((pr[0] + pr[1]) + (pr[2] + pr[3]));
                 uint32_t pf[4];
-                split_h2(pr[0], pr[1], pf[0], pf[1]);
-                split_h2(pr[2], pr[3], pf[2], pf[3]);
-#pragma unroll
-                for (int v = 0; v < NV; ++v)
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) o[v][e] *= es;
+                split_h2(pr[0] * kUp, pr[1] * kUp, pf[0], pf[1]);
+                split_h2(pr[2] * kUp, pr[3] * kUp, pf[2], pf[3]);
 #pragma unroll
                 for (int v = 0; v < NV; v += 2) {
                     uint32_t f[4];
                     const uint32_t c = uint32_t(v + (lane >> 4));
                     ldsm4t(f, vrow + (c >> 3) * BOX_BYTES + (((c & 7) ^ sw) << 4));
-                    mma16(o[v], pf, f[0], f[1]);
-                    mma16(o[v + 1], pf, f[2], f[3]);
+                    float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};
+                    mma16(d0, pf, f[0], f[1]);
+                    mma16(d1, pf, f[2], f[3]);
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        o[v][e] = fmaf(o[v][e], es, d0[e] + d0[e + 2]);
+                        o[v + 1][e] = fmaf(o[v + 1][e], es, d1[e] + d1[e + 2]);
+                    }
                 }
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // this warp may have written a row of the page
@@ -213,7 +250,7 @@ __global__ void __launch_bounds__(kBlock, HD == 64 ? 3 : 2) attn_decode_kernel(c
         if (lc == 0) { s_ml[warp][lr][0] = m; s_ml[warp][lr][1] = l; }
 #pragma unroll
         for (int v = 0; v < NV; ++v)
-            *reinterpret_cast<float2*>(s_acc + (warp * kHeads + lr) * HD + v * 8 + lc) = make_float2(o[v][0] + o[v][2], o[v][1] + o[v][3]);
+            *reinterpret_cast<float2*>(s_acc + (warp * kHeads + lr) * HD + v * 8 + lc) = make_float2(o[v][0] * (1.f / kUp), o[v][1] * (1.f / kUp));
         csync();
         for (int idx = threadIdx.x; idx < gc * HD; idx += kThreads) {
             const int g = idx / HD;
@@ -359,7 +396,8 @@ int32_t attn_decode(const AttnDecodeArgs& a, cudaStream_t st) {
     // ring depth: the pages a CTA will see, at most what lets three CTAs (two with wider heads) share an SM
     const int ctx = a.seq_len ? a.max_ctx : a.seq_len_host;
     const int pages_per_cta = ((ctx + FORGE_KV_PAGE - 1) / FORGE_KV_PAGE + a.splits - 1) / a.splits;
-    DecParams p{a, kLog2e / sqrtf(float(a.hd)), std::max(1, std::min(pages_per_cta, a.hd == 64 ? 4 : 2))};
+    const double scale = 1.4426950408889634 / std::sqrt(double(a.hd));   // log2 e / sqrt(head_dim)
+    DecParams p{a, float(scale), std::max(1, std::min(pages_per_cta, a.hd == 64 ? 4 : 2)), float(scale - double(float(scale)))};
     dim3 grid(a.splits, a.nkv, a.batch);
     const bool sw = a.window > 0;
     if (a.hd == 64) return sw ? launch_decode<64, true>(mk, mv, p, grid, st) : launch_decode<64, false>(mk, mv, p, grid, st);

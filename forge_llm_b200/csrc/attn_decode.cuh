@@ -20,6 +20,7 @@ struct DecParams {
     AttnDecodeArgs a;
     float scale;  // of the scores
     int stages;   // ring depth of this launch (<= kStages)
+    float scale_lo;   // what `scale` leaves of its exact value
 };
 
 #ifdef __CUDACC__

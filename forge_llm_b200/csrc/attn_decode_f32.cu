@@ -348,7 +348,7 @@ int32_t attn_decode_f32(const AttnDecodeArgs& a, cudaStream_t st) {
     // a CTA with one or two pages takes a ring of two; three CTAs per SM (two with 128-wide heads) share its shared memory with their merge buffers: a ring of 48 KB
     // each for 64- and 96-wide heads (3 and 2 pages of K and V), 64 KB (2 pages) for 128-wide
     const int fit = std::max(2, int((56u << 10) / (2u * FORGE_KV_PAGE * a.hd * sizeof(__half))));
-    DecParams p{a, 1.0f / sqrtf(float(a.hd)), pages_per_cta <= 2 ? 2 : std::min(kStages, fit)};
+    DecParams p{a, 1.0f / sqrtf(float(a.hd)), pages_per_cta <= 2 ? 2 : std::min(kStages, fit), 0.f};
     dim3 grid(a.splits, a.nkv, a.batch);
     const int group = a.nq / a.nkv;
     if (group == 1) return launch_f32_hd<1>(a.hd, a.window > 0, mk, mv, p, grid, st);

@@ -97,3 +97,34 @@ def test_steps_of_models_with_many_heads_per_kv_head(hd, nq, nkv):
     assert rel_l2(got, want) < 1e-3    # the prompt's queries and weights enter its products as plain fp16
     kv.close()
     gm.close()
+
+
+@pytest.mark.parametrize("hd,nq,nkv", [(64, 14, 2), (96, 6, 2), (128, 8, 1)])
+@pytest.mark.parametrize("q_scale,k_scale", [(1e-30, 1.0), (1e-3, 1e3), (1e2, 1e-2), (4e6, 1e-6), (1e7, 1e-7)])
+def test_queries_of_any_size(hd, nq, nkv, q_scale, k_scale):
+    """A query is an f32 number: its size may not cost bits, and a large one may not overflow."""
+    q, k, v = inputs(hd, nq, nkv, 700, q_scale, k_scale)
+    assert error(attend(q, k, v, 700), attend64(q, k, v, 700)) < 3e-6
+
+
+@pytest.mark.parametrize("hd,nq,nkv,seq", [(64, 32, 8, 8192), (64, 14, 2, 20000), (96, 128, 128, 4096), (128, 32, 32, 8192), (128, 16, 2, 8192)])
+def test_long_sums_keep_f32(hd, nq, nkv, seq):
+    """Thousands of weights of one size: what an f32 result owes.  A sum of independent roundings of 2^-24 stays below 2.5e-7; sums that a tensor core carries from
+    page to page lose a bit toward zero at every step and come to 3.5e-7 and more."""
+    q, k, v = inputs(hd, nq, nkv, seq, q_scale=0.1)
+    assert error(attend(q, k, v, seq), attend64(q, k, v, seq)) < 2.8e-7
+
+
+@pytest.mark.parametrize("hd,nq,nkv", [(64, 14, 2), (128, 32, 32)])
+@pytest.mark.parametrize("above", [5, 10, 14])
+def test_weights_beside_a_first_token_that_takes_almost_all(hd, nq, nkv, above):
+    """A first token whose score lies far above the others' and whose value is zero: the result is made of weights of e^-above, and each of them
+    still has the bits of an f32 number."""
+    seq = 1000
+    q, k, v = inputs(hd, nq, nkv, seq, q_scale=0.1)
+    q[:, 0] = 4.0
+    k[:, :, 0] = 0
+    k[0, :, :] = 0
+    k[0, :, 0] = above * hd ** 0.5 / 4
+    v[0] = 0
+    assert error(attend(q, k, v, seq), attend64(q, k, v, seq)) < 1e-6
