@@ -55,9 +55,49 @@ __device__ __forceinline__ float remote_f32(uint32_t addr) {
     return v;
 }
 
+// barrier of the consumers that also tells whether any of them says so
+__device__ __forceinline__ bool csync_or(bool x) {
+    uint32_t any;
+    asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 p, %1, 0;\nbar.red.or.pred q, 1, %2, p;\nselp.u32 %0, 1, 0, q;\n}" : "=r"(any) : "r"(uint32_t(x)), "n"(kThreads) : "memory");
+    return any != 0;
+}
+
+// One head's sums over the CTA's pages by f32 multiply-adds, a warp per head, from global memory.  Taken where a sum came out as NaN: the two parts of a
+// query or a weight meet an infinite key or value with a zero or with the other sign, where their sum would have given an infinity.
+template <int HD, bool SW>
+__device__ __noinline__ void plain_head(const AttnDecodeArgs& a, float scale, int b, int kvh, int head, int split, int n_ctx, int t_first, size_t row0, float* sums, float* ml) {
+    constexpr int D = HD / 32;
+    const int lane = threadIdx.x & 31, kvd = a.nkv * HD;
+    const int32_t* pt = a.page_table ? a.page_table + size_t(b) * a.pages_per_seq : nullptr;
+    float q[D], acc[D], m = -INFINITY, l = 0.f;
+#pragma unroll
+    for (int i = 0; i < D; ++i) { q[i] = a.q[(size_t(b) * a.nq + head) * HD + i * 32 + lane] * scale; acc[i] = 0.f; }
+    for (int lp = split; lp * FORGE_KV_PAGE < n_ctx; lp += a.splits) {
+        const size_t page = row0 + size_t(pt ? pt[lp] : lp) * FORGE_KV_PAGE;
+        for (int r = SW ? max(0, t_first - lp * FORGE_KV_PAGE) : 0; r < min(FORGE_KV_PAGE, n_ctx - lp * FORGE_KV_PAGE); ++r) {
+            const size_t at = (page + r) * kvd + size_t(kvh) * HD + lane;
+            float s = 0.f;
+#pragma unroll
+            for (int i = 0; i < D; ++i) s = fmaf(q[i], __half2float(a.k_pool[at + i * 32]), s);
+#pragma unroll
+            for (int x = 16; x > 0; x >>= 1) s += __shfl_xor_sync(0xffffffffu, s, x);
+            const float mn = fmaxf(m, s);
+            if (mn == -INFINITY) continue;
+            const float es = exp2_rel(m, mn), w = exp2_rel(s, mn);
+            m = mn;
+            l = l * es + w;
+#pragma unroll
+            for (int i = 0; i < D; ++i) acc[i] = acc[i] * es + w * __half2float(a.v_pool[at + i * 32]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < D; ++i) sums[i * 32 + lane] = acc[i];
+    if (lane == 0) { ml[0] = m; ml[1] = l; }
+}
+
 // SW: sliding-window instantiation (the full-attention one carries no window tests); CL: the splits are a cluster
 template <int HD, bool SW, bool CL>
-__global__ void __launch_bounds__(kBlock, HD == 64 ? 3 : 2) attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, DecParams p) {
+__global__ void __launch_bounds__(kBlock, HD == 64 ? 3 : 2) attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const __grid_constant__ DecParams p) {
     constexpr int BOXES = (HD + 63) / 64;                 // boxes of 64 dimensions (the second one of 96-wide heads is half zeros)
     constexpr int BOX_BYTES = FORGE_KV_PAGE * 128;
     constexpr int PAGE_BYTES = BOXES * BOX_BYTES;
@@ -252,6 +292,20 @@ __global__ void __launch_bounds__(kBlock, HD == 64 ? 3 : 2) attn_decode_kernel(c
         for (int v = 0; v < NV; ++v)
             *reinterpret_cast<float2*>(s_acc + (warp * kHeads + lr) * HD + v * 8 + lc) = make_float2(o[v][0] * (1.f / kUp), o[v][1] * (1.f / kUp));
         csync();
+        auto put = [&](int idx, float M, float A, float L) {
+            const int g = idx / HD;
+            if (a.splits == 1) {
+                store_out(a, (size_t(b) * a.nq + kvh * G + g0) * HD + idx, A * (1.0f / L));
+            } else if (CL) {
+                s_sum[g0 * HD + idx] = A;
+                if (idx % HD == 0) { s_cml[g0 + g][0] = M; s_cml[g0 + g][1] = L; }
+            } else {
+                float* w = a.ws + ((size_t(b) * a.nq + kvh * G + g0 + g) * a.splits + split) * (HD + 2);
+                w[2 + idx % HD] = A;
+                if (idx % HD == 0) { w[0] = M; w[1] = L; }
+            }
+        };
+        bool nan = false;
         for (int idx = threadIdx.x; idx < gc * HD; idx += kThreads) {
             const int g = idx / HD;
             float M = -INFINITY, A = 0.f, L = 0.f;
@@ -263,18 +317,16 @@ __global__ void __launch_bounds__(kBlock, HD == 64 ? 3 : 2) attn_decode_kernel(c
                 A += s_acc[w * kHeads * HD + idx] * f;
                 L += s_ml[w][g][1] * f;
             }
-            if (a.splits == 1) {
-                store_out(a, (size_t(b) * a.nq + kvh * G + g0) * HD + idx, A * (1.0f / L));
-            } else if (CL) {
-                s_sum[g0 * HD + idx] = A;
-                if (idx % HD == 0) { s_cml[g0 + g][0] = M; s_cml[g0 + g][1] = L; }
-            } else {
-                float* w = a.ws + ((size_t(b) * a.nq + kvh * G + g0 + g) * a.splits + split) * (HD + 2);
-                w[2 + idx % HD] = A;
-                if (idx % HD == 0) { w[0] = M; w[1] = L; }
-            }
+            nan |= A != A || L != L;
+            put(idx, M, A, L);
         }
-        csync();
+        if (csync_or(nan)) {
+            for (int g = warp; g < gc; g += kThreads / 32)
+                plain_head<HD, SW>(a, p.scale, b, kvh, kvh * G + g0 + g, split, n_ctx, t_first, seq_base, s_acc + g * HD, s_ml[0][g]);
+            csync();
+            for (int idx = threadIdx.x; idx < gc * HD; idx += kThreads) put(idx, s_ml[0][idx / HD][0], s_acc[idx], s_ml[0][idx / HD][1]);
+            csync();
+        }
     }
     if (CL && a.splits > 1) {
         // ---- the CTAs' parts become the result, each CTA finishing a share of it.  Only here, behind the last pass: until then the producer lane may be

@@ -128,3 +128,22 @@ def test_weights_beside_a_first_token_that_takes_almost_all(hd, nq, nkv, above):
     k[0, :, 0] = above * hd ** 0.5 / 4
     v[0] = 0
     assert error(attend(q, k, v, seq), attend64(q, k, v, seq)) < 1e-6
+
+
+@pytest.mark.parametrize("hd,nq,nkv,seq,window", [(64, 14, 2, 100, 0), (64, 12, 1, 3000, 0), (64, 8, 2, 9000, 700), (96, 6, 2, 700, 0), (128, 16, 16, 2000, 300), (128, 4, 2, 20000, 0)])
+def test_infinite_keys_and_values(hd, nq, nkv, seq, window):
+    """What f32 arithmetic gives: an infinite value reaches the result with its sign, a key whose score is minus infinity has no weight, one whose
+    score is plus infinity takes the row with it.  Rows and KV heads without one are as they would be."""
+    import torch
+    q, k, v = inputs(hd, nq, nkv, seq)
+    G = nq // nkv
+    v[seq - 9, 0, 5], v[seq - 70, 0, 6] = float("inf"), float("-inf")
+    v[seq - 1, 0, 7] = v[seq - 30, 0, 7] = float("inf")
+    k[seq - 20, nkv - 1, 3] = float("-inf")
+    if nkv > 1:   # the last KV head's first query: with a positive value there the key is ignored, with a negative one the row is lost
+        q[(nkv - 1) * G, 3] = q[(nkv - 1) * G, 3].abs()
+    got, want = attend(q, k, v, seq, window), attend64(q, k, v, seq, window)
+    assert torch.equal(got.isnan(), want.isnan())
+    assert torch.equal(got.isinf(), want.isinf()) and torch.equal(got[got.isinf()].sign().double(), want[want.isinf()].sign())
+    ok = want.isfinite()
+    assert ok.any() and error(got[ok], want[ok]) < 3e-6
