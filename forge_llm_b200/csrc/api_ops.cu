@@ -295,7 +295,7 @@ int32_t forge_attention_flash(float* out, const float* q, const uint16_t* k_cach
     FORGE_TRY(need_device());
     if (!out || !q || !k_cache || !v_cache || seq_len <= 0 || num_heads <= 0 || num_kv_heads <= 0) { set_error("bad argument to forge_attention_flash"); return FORGE_ERR_INVALID_ARG; }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    int splits = attn_decode_splits((seq_len + FORGE_KV_PAGE - 1) / FORGE_KV_PAGE, num_kv_heads, 148, head_dim, num_heads / num_kv_heads);
+    int splits = attn_decode_splits((seq_len + FORGE_KV_PAGE - 1) / FORGE_KV_PAGE, num_kv_heads, 148, head_dim);
     AsyncBuf ws(st), cnt(st);
     if (const size_t fl = attn_decode_ws_floats(1, num_heads, head_dim, splits)) {
         FORGE_CUDA(ws.alloc(sizeof(float) * fl));
@@ -345,7 +345,7 @@ int32_t forge_attention_sliding(float* out, const float* q, const uint16_t* k_ca
     FORGE_TRY(need_device());
     if (!out || !q || !k_cache || !v_cache || seq_len <= 0 || window <= 0 || num_heads <= 0 || num_kv_heads <= 0) { set_error("bad argument to forge_attention_sliding"); return FORGE_ERR_INVALID_ARG; }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    int splits = attn_decode_splits((seq_len + FORGE_KV_PAGE - 1) / FORGE_KV_PAGE, num_kv_heads, 148, head_dim, num_heads / num_kv_heads);
+    int splits = attn_decode_splits((seq_len + FORGE_KV_PAGE - 1) / FORGE_KV_PAGE, num_kv_heads, 148, head_dim, window);
     AsyncBuf ws(st), cnt(st);
     if (const size_t fl = attn_decode_ws_floats(1, num_heads, head_dim, splits)) {
         FORGE_CUDA(ws.alloc(sizeof(float) * fl));

@@ -13,8 +13,8 @@
 // error for scores around 1, 0.65 around 10; 8000 keys of one weight 1.6e-7, 3.8e-7 with sums carried through the tensor core).
 // A page costs a warp about forty tensor instructions at head_dim 64 whatever the group; with scores and sums
 // formed by fused multiply-adds (four heads per pass over the page) one page took 1.7 us.
-// The splits of a (sequence, KV head) are a cluster and merge through distributed shared memory; beyond eight splits (contexts past 128 pages) the
-// last CTA to finish merges partials from global memory (atomic ticket).  Every wait is bounded.
+// The splits of a (sequence, KV head) are a cluster and merge through distributed shared memory; more than eight (few KV heads over many
+// pages) leave partials in global memory, which the last CTA to finish merges (atomic ticket).  Every wait is bounded.
 #include <algorithm>
 #include <cmath>
 #include <mutex>
@@ -107,7 +107,6 @@ __global__ void __launch_bounds__(kBlock, HD == 64 ? 3 : 2) attn_decode_kernel(c
     float* s_acc = reinterpret_cast<float*>(ring + size_t(p.stages) * 2 * PAGE_BYTES);
     __shared__ uint64_t full_bar[kStages], empty_bar[kStages];
     __shared__ float s_ml[4][kHeads][2], s_cml[kMaxGroup][2];
-    __shared__ float s_fw[kMaxSplits][kMaxGroup];         // global merge: weight of split s for query head g
     __shared__ int s_last;
     const AttnDecodeArgs& a = p.a;
     pdl_trigger();
@@ -126,6 +125,9 @@ __global__ void __launch_bounds__(kBlock, HD == 64 ? 3 : 2) attn_decode_kernel(c
     const int32_t* pt = a.page_table ? a.page_table + size_t(b) * a.pages_per_seq : nullptr;
     const int n_ctx = a.seq_len ? a.seq_len[b] + 1 : a.seq_len_host;
     const int n_pages = (n_ctx + FORGE_KV_PAGE - 1) / FORGE_KV_PAGE;
+    // without a cluster, CTAs beyond the context's pages have no part in it: a launch's splits are those of the longest context that it may meet
+    const int splits = CL ? a.splits : min(a.splits, n_pages);
+    if (!CL && split >= splits) return;
     const int t_first = (SW && n_ctx > a.window) ? n_ctx - a.window : 0;  // sliding window: first position seen
     const size_t seq_base = a.page_table ? 0 : size_t(b) * a.max_ctx;  // contiguous: [batch][max_ctx][kvd]
 
@@ -294,7 +296,7 @@ __global__ void __launch_bounds__(kBlock, HD == 64 ? 3 : 2) attn_decode_kernel(c
         csync();
         auto put = [&](int idx, float M, float A, float L) {
             const int g = idx / HD;
-            if (a.splits == 1) {
+            if (splits == 1) {
                 store_out(a, (size_t(b) * a.nq + kvh * G + g0) * HD + idx, A * (1.0f / L));
             } else if (CL) {
                 s_sum[g0 * HD + idx] = A;
@@ -328,17 +330,17 @@ __global__ void __launch_bounds__(kBlock, HD == 64 ? 3 : 2) attn_decode_kernel(c
             csync();
         }
     }
-    if (CL && a.splits > 1) {
+    if (CL && splits > 1) {
         // ---- the CTAs' parts become the result, each CTA finishing a share of it.  Only here, behind the last pass: until then the producer lane may be
         // waiting for ring space, and a cluster waits for every thread that has not left
         cluster_sync();
-        const int items = G * HD, share = (items + a.splits - 1) / a.splits;
+        const int items = G * HD, share = (items + splits - 1) / splits;
         for (int idx = split * share + threadIdx.x; idx < min(items, (split + 1) * share); idx += kThreads) {
             const int g = idx / HD;
             float pm[kClusterSplits], pl[kClusterSplits], px[kClusterSplits], M = -INFINITY, A = 0.f, L = 0.f;
 #pragma unroll
             for (int s = 0; s < kClusterSplits; ++s) {
-                const bool on = s < a.splits;
+                const bool on = s < splits;
                 pm[s] = on ? remote_f32(cluster_addr(&s_cml[g][0], s)) : -INFINITY;
                 pl[s] = on ? remote_f32(cluster_addr(&s_cml[g][1], s)) : 0.f;
                 px[s] = on ? remote_f32(cluster_addr(s_sum + idx, s)) : 0.f;
@@ -355,60 +357,78 @@ __global__ void __launch_bounds__(kBlock, HD == 64 ? 3 : 2) attn_decode_kernel(c
         }
         cluster_sync();   // nobody leaves while its sums are read
     }
-    if (CL || a.splits == 1) return;
+    if (CL || splits == 1) return;
 
     // ---- last CTA of this (batch, kv head) merges the splits
     __threadfence();
     csync();
     if (threadIdx.x == 0) {
         int old = atomicAdd(a.counters + b * a.nkv + kvh, 1);
-        s_last = (old == a.splits - 1);
+        s_last = (old == splits - 1);
         if (s_last) a.counters[b * a.nkv + kvh] = 0;  // ready for the next launch
     }
     csync();
     if (!s_last) return;
     __threadfence();
+    // One round trip: a thread asks for its two columns of all splits, then the warps turn the splits' (max, sum) pairs into weights (lane = split)
+    float (*s_fw)[kMaxGroup] = reinterpret_cast<float (*)[kMaxGroup]>(s_acc);   // [split][head]: over the warps' sums, which are no longer needed
     const float* ws_kvh = a.ws + (size_t(b) * a.nq + size_t(kvh) * G) * a.splits * (HD + 2);
-    for (int g = warp; g < G; g += kThreads / 32) {
-        const float* w = ws_kvh + (size_t(g) * a.splits + lane) * (HD + 2);
-        const float m = lane < a.splits ? __ldcg(w) : -INFINITY;
-        const float l = lane < a.splits ? __ldcg(w + 1) : 0.f;
-        float M = m;
+    for (int i0 = 0; i0 < G * HD / 2; i0 += kThreads) {
+        const int idx = i0 + threadIdx.x;
+        const bool on = idx < G * HD / 2;
+        const int g = on ? idx / (HD / 2) : 0, d2 = on ? idx % (HD / 2) : 0;
+        const float* w0 = ws_kvh + size_t(g) * a.splits * (HD + 2) + 2 + 2 * d2;
+        float2 pa[kMaxSplits];
 #pragma unroll
-        for (int x = 16; x > 0; x >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, x));
-        const float wt = exp2_rel(m, M);
-        float L = l * wt;
+        for (int s = 0; s < kMaxSplits; ++s)
+            pa[s] = (on && s < splits) ? __ldcg(reinterpret_cast<const float2*>(w0 + size_t(s) * (HD + 2))) : make_float2(0.f, 0.f);
+        if (i0 == 0) {
+            for (int g2 = warp; g2 < G; g2 += kThreads / 32) {
+                const float* w = ws_kvh + (size_t(g2) * a.splits + lane) * (HD + 2);
+                const float m = lane < splits ? __ldcg(w) : -INFINITY;
+                const float l = lane < splits ? __ldcg(w + 1) : 0.f;
+                float M = m;
 #pragma unroll
-        for (int x = 16; x > 0; x >>= 1) L += __shfl_xor_sync(0xffffffffu, L, x);
-        s_fw[lane][g] = wt * (1.0f / L);
-    }
-    csync();
-    for (int idx = threadIdx.x; idx < G * HD; idx += kThreads) {
-        const int g = idx / HD;
-        const float* w0 = ws_kvh + size_t(g) * a.splits * (HD + 2) + 2 + idx % HD;
-        float A = 0.f;
-#pragma unroll 8
-        for (int s = 0; s < a.splits; ++s) A += __ldcg(w0 + size_t(s) * (HD + 2)) * s_fw[s][g];
-        store_out(a, (size_t(b) * a.nq + kvh * G) * HD + idx, A);
+                for (int x = 16; x > 0; x >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, x));
+                const float wt = exp2_rel(m, M);
+                float L = l * wt;
+#pragma unroll
+                for (int x = 16; x > 0; x >>= 1) L += __shfl_xor_sync(0xffffffffu, L, x);
+                s_fw[lane][g2] = wt * (1.0f / L);
+            }
+            csync();
+        }
+        float2 A = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int s = 0; s < kMaxSplits; ++s) {
+            const float wt = s < splits ? s_fw[s][g] : 0.f;
+            A.x += pa[s].x * wt;
+            A.y += pa[s].y * wt;
+        }
+        if (on) store_out2(a, (size_t(b) * a.nq + size_t(kvh) * G + g) * HD + 2 * d2, A);
     }
 }
 
 }  // namespace
 
-// Context splits for `groups` = batch * kv_heads independent (sequence, KV head) pairs over `pages` pages.  CTAs run in rounds over the resident slots; a
-// CTA costs a fixed share (query, merge) and a share per page, so the splits are those whose rounds are done first: one sequence takes
-// eight, sixteen sequences of 32 KV heads one.  More than a cluster's eight only where a CTA would still walk sixteen pages.
-int attn_decode_splits(int pages, int groups, int sms, int hd, int) {
-    const int per_sm = hd == 64 ? 3 : 2;
-    const long slots = long(sms) * per_sm;
-    const int top = pages > 16 * kClusterSplits ? kMaxSplits : kClusterSplits, smax = std::max(1, std::min(pages, top));
-    const double page = hd == 64 ? 0.3 : 0.5, fixed = 1.5;
+// Context splits for `groups` = batch * kv_heads independent (sequence, KV head) pairs over `pages` pages, by what a launch took (cold caches, us): a CTA
+// 2.4 + 0.62 a page at 64 dimensions, 3.2 + 0.78 at 96 and 128, its pages longer where an SM's CTAs share it, in rounds over the resident CTAs; the meeting of
+// a cluster 1.8 (2.2), that through global memory 2.2 + 0.063 a split (3.3 + 0.094).  Beyond a cluster's eight only sixteen and 32: in between, CTAs of
+// unequal lengths were slower than the better of the two.  So 32 heads over 8 KV heads of 64 take 7.0 us over 25 pages with eight splits (sixteen
+// 6.6), 9.3 over 64 pages (sixteen 8.0, 32 7.8), 14.2 over 128 (10.3, 9.7); sixteen sequences of 32 KV heads take one.
+int attn_decode_splits(int pages, int groups, int sms, int hd, int window) {
+    if (window > 0) pages = std::min(pages, (window + FORGE_KV_PAGE - 2) / FORGE_KV_PAGE + 1);   // those that a window can touch
+    const bool wide = hd > 64;
+    const long slots = long(sms) * (wide ? 2 : 3);
+    const double fixed = wide ? 3.2 : 2.4, page = wide ? 0.78 : 0.62;
     int best = 1;
     double best_cost = 1e30;
-    for (int s = 1; s <= smax; ++s) {
-        const long rounds = (long(groups) * s + slots - 1) / slots;
-        const double cost = double(rounds) * (fixed + (s > 1 ? 0.5 : 0.0) + (s > kClusterSplits ? 1.0 : 0.0) + page * ((pages + s - 1) / s));
-        if (cost < best_cost - 1e-12) { best_cost = cost; best = s; }
+    for (int s = 1; s <= std::min(pages, kMaxSplits); s = s < kClusterSplits ? s + 1 : 2 * s) {
+        const long ctas = long(groups) * s, rounds = (ctas + slots - 1) / slots;
+        const double load = std::max(1.0, 0.85 * double(std::min(ctas, slots)) / sms);
+        const double meeting = s == 1 ? 0.0 : s <= kClusterSplits ? (wide ? 2.2 : 1.8) : wide ? 3.3 + 0.094 * s : 2.2 + 0.063 * s;
+        const double cost = double(rounds) * (fixed + page * load * ((pages + s - 1) / s)) + meeting;
+        if (cost < best_cost + 1e-9) { best_cost = cost; best = s; }   // of equals the larger: more of its CTAs have a page less
     }
     return best;
 }
@@ -445,7 +465,8 @@ int32_t attn_decode(const AttnDecodeArgs& a, cudaStream_t st) {
         FORGE_TRY(make_kv_map(&mk, a.k_pool, a.hd, a.nkv, rows));
         FORGE_TRY(make_kv_map(&mv, a.v_pool, a.hd, a.nkv, rows));
     }
-    // ring depth: the pages a CTA will see, at most what lets three CTAs (two with wider heads) share an SM
+    // ring depth: the pages a CTA will see, at most what lets three CTAs (two with wider heads) share an SM: 64-wide heads four stages of 16 KB and 8 KB of
+    // sums (with the second pass's 4 KB more two CTAs)
     const int ctx = a.seq_len ? a.max_ctx : a.seq_len_host;
     const int pages_per_cta = ((ctx + FORGE_KV_PAGE - 1) / FORGE_KV_PAGE + a.splits - 1) / a.splits;
     const double scale = 1.4426950408889634 / std::sqrt(double(a.hd));   // log2 e / sqrt(head_dim)
@@ -528,7 +549,7 @@ extern "C" int32_t forge_attention_flash_static(float* out, const float* q, cons
     StaticScratch* sc = nullptr;
     FORGE_TRY(static_scratch(&sc));
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int splits = std::min(kStaticMaxSplits, attn_decode_splits((seq_len + FORGE_KV_PAGE - 1) / FORGE_KV_PAGE, num_kv_heads, 148, head_dim, num_heads / num_kv_heads));
+    const int splits = std::min(kStaticMaxSplits, attn_decode_splits((seq_len + FORGE_KV_PAGE - 1) / FORGE_KV_PAGE, num_kv_heads, 148, head_dim));
     // the tickets must start at zero; the partials are fully rewritten by every call that reads them
     FORGE_CUDA(cudaMemsetAsync(sc->counters, 0, sizeof(int) * num_kv_heads, st));
     AttnDecodeArgs a{out, q, reinterpret_cast<const __half*>(k_cache), reinterpret_cast<const __half*>(v_cache), nullptr, 0, nullptr,

@@ -273,9 +273,9 @@ struct AttnDecodeArgs {
     // tensor maps are then those of the _f32 functions
     bool f32 = false;
 };
-// context splits for `groups` = batch * kv_heads independent (sequence, KV head) pairs over `pages` pages.  Up to eight need no
+// context splits for `groups` = batch * kv_heads independent (sequence, KV head) pairs over `pages` pages (window: as in the arguments).  Up to eight need no
 // workspace (attn_decode_ws_floats is 0): a.ws and a.counters may then be null
-int attn_decode_splits(int pages, int groups, int sms, int hd, int heads_per_group);
+int attn_decode_splits(int pages, int groups, int sms, int hd, int window = 0);
 size_t attn_decode_ws_floats(int batch, int nq, int hd, int splits);
 int attn_decode_f32_splits(int pages, int groups, int sms, int hd, int heads_per_group);
 size_t attn_decode_f32_ws_floats(int batch, int nq, int hd, int splits);

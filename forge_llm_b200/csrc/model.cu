@@ -333,7 +333,7 @@ int launch_splits(const ForgeModel* m, const ForgeKV* kv, int batch) {
     if (batch >= kv->batch || m->any_kquant) return kv->splits;
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device);
-    const int s = attn_decode_splits(kv->pages_per_seq, batch * m->nkv, sms, m->hd, m->nq / m->nkv);
+    const int s = attn_decode_splits(kv->pages_per_seq, batch * m->nkv, sms, m->hd, m->cfg.sliding_window);
     return attn_decode_ws_floats(1, 1, 1, s) ? kv->splits : s;
 }
 int32_t ensure_batch_buffers(ForgeModel* m) {
@@ -940,7 +940,8 @@ int32_t forge_kv_create_pool(ForgeModel* m, int32_t pool_tokens, int32_t max_seq
     if (!m->stack) {
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device);
-    kv->splits = (m->any_kquant ? attn_decode_f32_splits : attn_decode_splits)(kv->pages_per_seq, batch * m->nkv, sms, m->hd, m->nq / m->nkv);
+    kv->splits = m->any_kquant ? attn_decode_f32_splits(kv->pages_per_seq, batch * m->nkv, sms, m->hd, m->nq / m->nkv)
+                               : attn_decode_splits(kv->pages_per_seq, batch * m->nkv, sms, m->hd, m->cfg.sliding_window);
     if (cudaMalloc(&kv->attn_ws, sizeof(float) * (m->any_kquant ? attn_decode_f32_ws_floats : attn_decode_ws_floats)(batch, m->nq, m->hd, kv->splits)) != cudaSuccess ||
         cudaMalloc(&kv->attn_counters, sizeof(int) * batch * m->nkv) != cudaSuccess) { set_error("attention workspace allocation failed"); return fail(FORGE_ERR_CUDA); }
     cudaMemsetAsync(kv->attn_counters, 0, sizeof(int) * batch * m->nkv, m->stream);
