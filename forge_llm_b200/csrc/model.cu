@@ -328,14 +328,6 @@ struct PrefillToken { int seq; const uint32_t* tok; bool head; float* trace_dst;
 // order this follows).  Activations are packed as fp16 hi/lo fragments in front of each product (with the RMSNorm or
 // SiLU*up that feeds it), bias + RoPE + cache append and the single-query attention run per sequence.
 constexpr int kBatchGroup = 16;
-// splits of the decode attention for the sequences of one launch; the workspace of more than eight was made for all of the cache's
-int launch_splits(const ForgeModel* m, const ForgeKV* kv, int batch) {
-    if (batch >= kv->batch || m->any_kquant) return kv->splits;
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device);
-    const int s = attn_decode_splits(kv->pages_per_seq, batch * m->nkv, sms, m->hd, m->cfg.sliding_window);
-    return attn_decode_ws_floats(1, 1, 1, s) ? kv->splits : s;
-}
 int32_t ensure_batch_buffers(ForgeModel* m) {
     if (m->d_bact) return FORGE_OK;
     const int maxK = std::max({m->h, m->qk, m->ff});
@@ -427,7 +419,7 @@ int32_t decode_launches_batched(ForgeModel* m, ForgeKV* kv, int batch, bool gree
         FORGE_TRY(qkv_post_rows(m->p_qkv, n, L.qkv_bias, m->rope, m->d_q, kp, vp, kv->d_page_table, kv->d_seq_len, kv->pages_per_seq,
                                 m->qk, m->kv, m->hd, st));
         AttnDecodeArgs da{m->d_attn, m->d_q, kp, vp, kv->d_page_table, kv->pages_per_seq, kv->d_seq_len, 0,
-                          n, m->nq, m->nkv, m->hd, kv->max_seq, kv->attn_ws, kv->attn_counters, launch_splits(m, kv, n), c.sliding_window};
+                          n, m->nq, m->nkv, m->hd, kv->max_seq, kv->attn_ws, kv->attn_counters, kv->splits[n], c.sliding_window};
         da.map_k = kv->k_map; da.map_v = kv->v_map; da.row_base = int(size_t(l) * kv->num_pages * FORGE_KV_PAGE); da.err = m->d_err; da.f32 = m->any_kquant;
         FORGE_TRY(attn_decode(da, st));
         FORGE_TRY(batched_row_sliced(m, L.o_t, m->d_attn, m->qk, PLAIN, n, &sums, &pending, st));
@@ -466,7 +458,7 @@ int32_t decode_launches_gemm(ForgeModel* m, ForgeKV* kv, int batch, bool greedy,
         FORGE_TRY(qkv_post_rows(qks > 1 ? m->p_qkv_parts : m->p_qkv, n, L.qkv_bias, m->rope, m->d_q, kp, vp, kv->d_page_table, kv->d_seq_len,
                                 kv->pages_per_seq, m->qk, m->kv, m->hd, st, qks, qstride));
         AttnDecodeArgs da{m->d_attn, m->d_q, kp, vp, kv->d_page_table, kv->pages_per_seq, kv->d_seq_len, 0,
-                          n, m->nq, m->nkv, m->hd, kv->max_seq, kv->attn_ws, kv->attn_counters, launch_splits(m, kv, n), c.sliding_window};
+                          n, m->nq, m->nkv, m->hd, kv->max_seq, kv->attn_ws, kv->attn_counters, kv->splits[n], c.sliding_window};
         da.map_k = kv->k_map; da.map_v = kv->v_map; da.row_base = int(size_t(l) * kv->num_pages * FORGE_KV_PAGE); da.err = m->d_err; da.f32 = m->any_kquant;
         da.out16 = m->p_attn16; da.out16_lo = alo;   // straight into the o-projection's operand form
         FORGE_TRY(attn_decode(da, st));
@@ -542,7 +534,7 @@ int32_t decode_launches(ForgeModel* m, ForgeKV* kv, int batch, bool greedy, bool
             FORGE_TRY(gemv_tc(L.v_t, EPI_QKV, v, m->split, m->d_err, st));
         }
         AttnDecodeArgs da{m->d_attn, m->d_q, kp, vp, page_table, kv->pages_per_seq, seq_len, 0,
-                          batch, m->nq, m->nkv, m->hd, kv->max_seq, kv->attn_ws, kv->attn_counters, launch_splits(m, kv, batch), c.sliding_window};
+                          batch, m->nq, m->nkv, m->hd, kv->max_seq, kv->attn_ws, kv->attn_counters, kv->splits[batch], c.sliding_window};
         da.map_k = kv->k_map; da.map_v = kv->v_map; da.row_base = int(size_t(l) * kv->num_pages * FORGE_KV_PAGE); da.err = m->d_err; da.f32 = m->any_kquant;
         FORGE_TRY(attn_decode(da, st));
         GemvArgs o;
@@ -940,9 +932,15 @@ int32_t forge_kv_create_pool(ForgeModel* m, int32_t pool_tokens, int32_t max_seq
     if (!m->stack) {
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device);
-    kv->splits = m->any_kquant ? attn_decode_f32_splits(kv->pages_per_seq, batch * m->nkv, sms, m->hd, m->nq / m->nkv)
-                               : attn_decode_splits(kv->pages_per_seq, batch * m->nkv, sms, m->hd, m->cfg.sliding_window);
-    if (cudaMalloc(&kv->attn_ws, sizeof(float) * (m->any_kquant ? attn_decode_f32_ws_floats : attn_decode_ws_floats)(batch, m->nq, m->hd, kv->splits)) != cudaSuccess ||
+    // by the sequences of a launch, with the largest workspace that any of them needs (the f32 form keeps the cache's: its sums stay in their order)
+    kv->splits.assign(size_t(batch) + 1, 1);
+    size_t ws = 0;
+    for (int n = 1; n <= batch; ++n) {
+        kv->splits[n] = m->any_kquant ? attn_decode_f32_splits(kv->pages_per_seq, batch * m->nkv, sms, m->hd, m->nq / m->nkv)
+                                      : attn_decode_splits(kv->pages_per_seq, n * m->nkv, sms, m->hd, m->cfg.sliding_window);
+        ws = std::max(ws, (m->any_kquant ? attn_decode_f32_ws_floats : attn_decode_ws_floats)(n, m->nq, m->hd, kv->splits[n]));
+    }
+    if (cudaMalloc(&kv->attn_ws, sizeof(float) * ws) != cudaSuccess ||
         cudaMalloc(&kv->attn_counters, sizeof(int) * batch * m->nkv) != cudaSuccess) { set_error("attention workspace allocation failed"); return fail(FORGE_ERR_CUDA); }
     cudaMemsetAsync(kv->attn_counters, 0, sizeof(int) * batch * m->nkv, m->stream);
     }

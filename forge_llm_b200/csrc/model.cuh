@@ -90,7 +90,8 @@ struct ForgeKV {
     size_t layer_stride = 0;  // halfs per layer pool
     int32_t* d_page_table = nullptr; int32_t* d_seq_len = nullptr;
     std::vector<int32_t> h_page_table; std::vector<int> free_pages; std::vector<int> pages_used; std::vector<int> len;
-    float* attn_ws = nullptr; int* attn_counters = nullptr; int splits = 1;
+    float* attn_ws = nullptr; int* attn_counters = nullptr;
+    std::vector<int> splits;       // context splits of the decode attention, by the sequences of a launch
     StackCache* stack = nullptr;   // cache rows and states of a layer-list model (then k_pool and v_pool stay empty)
     int slot0 = 0;                 // of a view of single sequences: the first one's state slot
     std::vector<char> lost;        // sequences whose recurrent state a failed step has left undefined

@@ -147,3 +147,29 @@ def test_infinite_keys_and_values(hd, nq, nkv, seq, window):
     assert torch.equal(got.isinf(), want.isinf()) and torch.equal(got[got.isinf()].sign().double(), want[want.isinf()].sign())
     ok = want.isfinite()
     assert ok.any() and error(got[ok], want[ok]) < 3e-6
+
+
+def test_steps_of_fewer_sequences_than_the_cache_holds():
+    """A long cache of many sequences, stepped by one and by three of them: their launches take more context splits than one of all sequences
+    would, and the logits are those of a cache of their own."""
+    from forge_llm_b200 import configs, runtime, synth
+    c = configs.tiny(8, hd=64, nq=4, nkv=1, layers=1)
+    gm = runtime.Model(c, synth.make_weights_bin(c))
+    prompts = [synth.prompt_tokens(c, n, seed=n) for n in (4000, 2500, 130)]
+    own = []
+    for p in prompts:
+        kv = gm.new_cache(max_seq=4096)
+        gm.forward_prefill(p, kv, want_logits=False)
+        own.append(gm.forward(int(p[0]), kv))
+        kv.close()
+    kv = gm.new_cache(max_seq=4096, batch=64)
+    for i, p in enumerate(prompts):
+        gm.forward_prefill(p, kv, seq=i, want_logits=False)
+    got = gm.forward_batch([int(p[0]) for p in prompts], kv)
+    for a, b in zip(got, own):
+        assert rel_l2(a, b) < 1e-4    # products of several rows round otherwise
+    kv.reset()
+    gm.forward_prefill(prompts[0], kv, want_logits=False)
+    assert rel_l2(gm.forward(int(prompts[0][0]), kv), own[0]) < 1e-5
+    kv.close()
+    gm.close()
