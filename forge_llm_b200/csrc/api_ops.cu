@@ -14,7 +14,9 @@ namespace {
 
 // Scratch of the operator calls comes from a stream-ordered pool of this library's own.  The default pool gives memory back at every
 // synchronisation, and mapping it again cost a caller who waits for each call 0.5 ms for eight products; this one keeps up to kPoolKeep bytes per device
-// until the last packed projection is destroyed.  The pool itself orders reuse between streams and threads.
+// while a packed projection lives (what goes beyond them is given back at synchronisations).  Without one it keeps nothing, as the default pool does: a
+// caller of raw-block products or of the attention alone has no handle whose end could give the memory back.  The pool itself orders reuse between
+// streams and threads.
 constexpr uint64_t kPoolKeep = 256ull << 20;
 constexpr int kMaxDevices = 64;
 std::mutex g_pool_mutex;
@@ -33,7 +35,7 @@ cudaError_t scratch_pool(cudaMemPool_t* out) {
         props.location.id = dev;
         cudaMemPool_t pool = nullptr;
         if (cudaError_t e = cudaMemPoolCreate(&pool, &props)) return e;
-        uint64_t keep = kPoolKeep;
+        uint64_t keep = g_packed_live ? kPoolKeep : 0;
         if (cudaError_t e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep)) { cudaMemPoolDestroy(pool); return e; }
         g_pool[dev] = pool;
     }
@@ -42,9 +44,15 @@ cudaError_t scratch_pool(cudaMemPool_t* out) {
 }
 void count_packed(int by) {
     std::lock_guard<std::mutex> lock(g_pool_mutex);
+    const bool was = g_packed_live > 0;
     g_packed_live += by;
-    if (g_packed_live == 0)
-        for (cudaMemPool_t p : g_pool) if (p) cudaMemPoolTrimTo(p, 0);   // what is in use stays
+    if ((g_packed_live > 0) == was) return;
+    uint64_t keep = was ? 0 : kPoolKeep;
+    for (cudaMemPool_t p : g_pool) {
+        if (!p) continue;
+        cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+        if (was) cudaMemPoolTrimTo(p, 0);   // what is in use stays until it is free
+    }
 }
 
 struct AsyncBuf {

@@ -118,7 +118,8 @@ int32_t forge_matmul_vec_q6_k(float* out, int32_t m, const float* in, const uint
 /* The same products on a weight repacked once: forge_packed_create converts raw GGUF blocks
  * (device pointer, [N][K/32][block]) into the kernels' aligned layouts (same bytes per weight),
  * forge_matmul_mat_packed then runs without any per-call repacking or allocation for m < 8
- * (the `Weights` struct of the generated module, E:3875-3939, plays this role there). */
+ * (the `Weights` struct of the generated module, E:3875-3939, plays this role there).  While a packed weight lives the
+ * library keeps up to 256 MB of scratch of the operator calls per device; with the last one they are given back. */
 typedef struct ForgePacked ForgePacked;
 int32_t forge_packed_create(int32_t quant, const uint8_t* w, int32_t K, int32_t N, void* stream, ForgePacked** out);
 void forge_packed_destroy(ForgePacked* w);

@@ -291,3 +291,28 @@ def test_argmax_last_index_on_ties(L, oracle):
         check(lib.forge_argmax(res.data_ptr(), dx.data_ptr(), n, None))
         _sync()
         assert int(res.item()) == oracle.argmax(x) == n - 2
+
+
+def test_scratch_of_raw_block_products_is_given_back():
+    """Scratch stays with the library only while a packed weight lives: a caller of raw-block products has nothing that could end, and finds the device's
+    memory as it was once it has waited for its calls."""
+    import torch
+    from forge_llm_b200 import synth
+    from forge_llm_b200._lib import check, lib
+    rng = np.random.default_rng(5)
+    m, K, N = 4096, 4096, 256      # 64 MB of fp16 parts
+    w, x = dev(synth.quantize(8, rng.standard_normal((N, K), dtype=np.float32))), torch.randn(m, K, device="cuda")
+    out = torch.empty(m, N, device="cuda")
+
+    def call():
+        check(lib.forge_matmul_mat_q8_0(out.data_ptr(), m, x.data_ptr(), w.data_ptr(), K, N, None))
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    pk = C.c_void_p()
+    check(lib.forge_packed_create(8, w.data_ptr(), K, N, None, C.byref(pk)))
+    kept = call()                  # kernels loaded, scratch kept
+    lib.forge_packed_destroy(pk)
+    free = torch.cuda.mem_get_info()[0]
+    assert free >= kept + (64 << 20)
+    assert call() >= free - (8 << 20)      # and nothing is kept by a call behind the last destroy
