@@ -63,7 +63,8 @@ __device__ __forceinline__ bool csync_or(bool x) {
 }
 
 // One head's sums over the CTA's pages by f32 multiply-adds, a warp per head, from global memory.  Taken where a sum came out as NaN: the two parts of a
-// query or a weight meet an infinite key or value with a zero or with the other sign, where their sum would have given an infinity.
+// query or a weight meet an infinite key or value with a zero or with the other sign, where their sum would have given an infinity; or a page did not
+// come within the wait's limit.
 template <int HD, bool SW>
 __device__ __noinline__ void plain_head(const AttnDecodeArgs& a, float scale, int b, int kvh, int head, int split, int n_ctx, int t_first, size_t row0, float* sums, float* ml) {
     constexpr int D = HD / 32;
@@ -196,7 +197,10 @@ __global__ void __launch_bounds__(kBlock, HD == 64 ? 3 : 2) attn_decode_kernel(c
             if (SW && (lp + 1) * FORGE_KV_PAGE <= t_first) continue;  // the whole page lies before the window
             const int t0 = lp * FORGE_KV_PAGE + warp * 16;            // the warp's sixteen keys
             const int st = pi % p.stages;
-            if (!mbar_wait(&full_bar[st], (pi / p.stages) & 1) && a.err) atomicExch(a.err, 1);
+            if (!mbar_wait(&full_bar[st], (pi / p.stages) & 1)) {   // a session's call fails; an operator call has no such word, and its sums are formed again
+                if (a.err) atomicExch(a.err, 1);
+                l = NAN;
+            }
             unsigned char* const ks = ring + size_t(st) * 2 * PAGE_BYTES + warp * 16 * 128;
             if (t0 < n_ctx && (!SW || t0 + 16 > t_first)) {
                 if (n_ctx - 1 - t0 < 16) {
