@@ -173,3 +173,14 @@ def test_steps_of_fewer_sequences_than_the_cache_holds():
     assert rel_l2(gm.forward(int(prompts[0][0]), kv), own[0]) < 1e-5
     kv.close()
     gm.close()
+
+
+@pytest.mark.parametrize("hd,nq,nkv", [(64, 7, 1), (64, 28, 2), (96, 8, 1), (96, 6, 6), (96, 20, 2), (128, 14, 2), (128, 16, 1)])
+@pytest.mark.parametrize("seq,window", [(40, 17), (129, 64), (130, 65), (1000, 500), (2500, 2400), (8300, 1), (8300, 4100), (20000, 19937)])
+def test_windows_with_every_group(hd, nq, nkv, seq, window):
+    """Windows that begin within a warp's keys, at a page and beyond whole splits, for one to sixteen query heads per KV head: what lies in front of them
+    has no weight, whatever it holds."""
+    q, k, v = inputs(hd, nq, nkv, seq)
+    want = attend64(q, k, v, seq, window)
+    k[:seq - window], v[:seq - window] = float("nan"), float("inf")
+    assert error(attend(q, k, v, seq, window), want) < 3e-6
