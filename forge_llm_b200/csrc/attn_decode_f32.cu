@@ -1,7 +1,7 @@
 // Single-query decode attention with scores and sums by f32 multiply-adds: what models with K-quant projections take.  Their products round every
-// row to 8 bits first, so the last bit of an attention result can move a whole step of that rounding; queries and probabilities therefore keep all 24
-// bits here and the order of the sums is fixed.  attn_decode.cu, on tensor cores, is the faster one where results go on as they are (one sequence of
-// 32 heads over 8 KV heads of 64: 8.3 us there, 9.9 here).
+// row to 8 bits first, so a last bit of an attention result that comes out otherwise can move a whole step of that rounding: the order of the sums is
+// part of what these models give, and it is fixed here.  attn_decode.cu, on tensor cores, is nearer to the exact result and the faster one where results go on
+// as they are (one sequence of 32 heads over 8 KV heads of 64, 1560 positions: 6.9 us there, 7.7 here).
 // HBM-bound on K/V: the context is split over CTAs (split-KV); a producer lane pulls the CTA's pages - 64 rows of one
 // KV head, K and V - into a ring of shared-memory stages with 3-D tiled TMA copies (cp.async.bulk.tensor, mbarrier
 // completion; the tensor map spans this GPU's own pool), so the bytes in flight do not depend on registers or on
