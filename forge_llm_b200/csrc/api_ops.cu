@@ -59,6 +59,10 @@ struct AsyncBuf {
     void* p = nullptr; cudaStream_t st;
     explicit AsyncBuf(cudaStream_t s) : st(s) {}
     cudaError_t alloc(size_t bytes) {
+        // what is allocated under capture belongs to the graph and to no pool, and a capture may not create one
+        cudaStreamCaptureStatus capture;
+        if (cudaError_t e = cudaStreamIsCapturing(st, &capture)) return e;
+        if (capture != cudaStreamCaptureStatusNone) return cudaMallocAsync(&p, bytes ? bytes : 1, st);
         cudaMemPool_t pool = nullptr;
         if (cudaError_t e = scratch_pool(&pool)) return e;
         return cudaMallocFromPoolAsync(&p, bytes ? bytes : 1, pool, st);

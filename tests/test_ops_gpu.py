@@ -316,3 +316,41 @@ def test_scratch_of_raw_block_products_is_given_back():
     free = torch.cuda.mem_get_info()[0]
     assert free >= kept + (64 << 20)
     assert call() >= free - (8 << 20)      # and nothing is kept by a call behind the last destroy
+
+
+CAPTURE = """
+import ctypes as C
+import numpy as np
+import torch
+from forge_llm_b200 import synth
+from forge_llm_b200._lib import check, lib
+K, N, m = 1024, 512, 40
+w = torch.from_numpy(synth.quantize(8, np.random.default_rng(1).standard_normal((N, K), dtype=np.float32))).cuda()
+x, out, other = torch.randn(m, K, device="cuda"), torch.zeros(m, N, device="cuda"), torch.zeros(m, N, device="cuda")
+pk = C.c_void_p()
+check(lib.forge_packed_create(8, w.data_ptr(), K, N, None, C.byref(pk)))
+torch.cuda.synchronize()
+s, g = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+with torch.cuda.graph(g, stream=s):
+    check(lib.forge_matmul_mat_packed(out.data_ptr(), m, x.data_ptr(), pk, s.cuda_stream))
+torch.cuda.synchronize()
+assert out.eq(0).all()
+check(lib.forge_matmul_mat_packed(other.data_ptr(), m, x.data_ptr(), pk, None))
+torch.cuda.synchronize()
+assert other.ne(0).any()
+for _ in range(2):
+    out.zero_()
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, other)
+"""
+
+
+def test_first_scratch_of_a_process_under_capture():
+    """A call whose scratch is the process's first, on a stream that is being captured: its graph gives what the call gives."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    done = subprocess.run([sys.executable, "-c", CAPTURE], cwd=root, capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]
