@@ -309,11 +309,17 @@ int32_t attn_prefill(const AttnPrefillArgs& a, cudaStream_t st);
 int32_t gemm_f16a(float* out, const __half* A, const __half* Alo, const QWeight& w, int m, const float* resid, int* err, cudaStream_t st);
 int32_t gemm_f16a_mma(float* out, const __half* A, const __half* Alo, const QWeight& w, int m, const float* resid, cudaStream_t st);
 bool gemm_tc5_supported(const QWeight& w);
-// ksplit > 1: K slice z leaves its partial product (no residual) at out + z * part_stride; the caller adds the slices
+// ksplit > 1: the K slices leave *parts partial products (ksplit of them where parts is null; no residual) at out + z * part_stride; the caller adds them
 // act_hi != null (gate/up product, rows 2j = gate_j, 2j + 1 = up_j, one K slice): the epilogue stores SiLU(gate) * up as
 // fp16 hi (+ lo) rows [m][N / 2] and `out` is not written
 int32_t gemm_tc5(float* out, const __half* A, const __half* Alo, const QWeight& w, int m, const float* resid, int* err, cudaStream_t st,
-                 int ksplit = 1, size_t part_stride = 0, __half* act_hi = nullptr, __half* act_lo = nullptr);
+                 int ksplit = 1, size_t part_stride = 0, __half* act_hi = nullptr, __half* act_lo = nullptr, int* parts = nullptr);
 int gemm_tc5_ksplit(const QWeight& w);
+// The same product on CTA pairs (gemm_pair.cu; Q8_0 / Q4_0, split precision): tokens per tile, partial outputs part_stride apart that remain to be added, pairs
+// launched, and the microseconds that this should take.  K runs as ksplit slices; parts_only != 0 asks for that many partial outputs
+struct PairPlan { int nt = 0, parts = 1, pairs = 0; double cost = 0; };
+PairPlan gemm_pair_plan(const QWeight& w, int m, int ksplit, int parts_only, int sms);
+int32_t gemm_pair(float* out, const __half* A, const __half* Alo, const QWeight& w, int m, const float* resid, int* err, cudaStream_t st, const PairPlan& plan, int ksplit,
+                  size_t part_stride, __half* act_hi, __half* act_lo);
 
 }  // namespace forge

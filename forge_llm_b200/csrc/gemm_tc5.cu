@@ -1,6 +1,7 @@
 // Prefill GEMM on the 5th-generation tensor cores (tcgen05 + TMEM): out[m][N] = A[m][K] x W[N][K]^T with W
 // streamed as Q8_0 / Q4_0 blocks and dequantised on the fly (replaces matmul_mat_q8_0_KxN /
-// matmul_mat_q4_0_KxN, crates/forgellm-codegen-cpu/src/emit.rs:2278-2299 and :3792-3813).
+// matmul_mat_q4_0_KxN, crates/forgellm-codegen-cpu/src/emit.rs:2278-2299 and :3792-3813): one CTA per tile, for single products (one fp16 pass) and for
+// K-quant rows.  Split-precision products of more than 32 rows take gemm_pair.cu.
 //
 // CTA tile: 128 weight rows (MMA M) x NT tokens (MMA N = 128, 192 or 256), K step 64.  The dequantised weight
 // tile is the A operand and lives in TENSOR memory; the activation tile is the B operand in shared memory;
@@ -28,11 +29,14 @@
 #include <cstring>
 
 #include "common.cuh"
+#include "gemm_tc5.cuh"
 #include "tc5.cuh"
 
 namespace forge {
 
 namespace {
+
+using namespace tc5w;
 
 constexpr int BK = 64;  // K step: one 128-byte swizzle row of fp16
 constexpr int kThreads = 320;
@@ -78,35 +82,6 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-struct Tc5Params {
-    float* out; const float* resid;
-    const uint8_t* qs; const __half* d; const float4* sf;
-    int m, N, K;
-    int* err;
-    int ksplit;            // K slices (grid.z); slice z leaves its partial product at out + z * part_stride
-    size_t part_stride;
-    // gate/up product (weight rows 2j = gate_j, 2j + 1 = up_j): when act_hi is set the epilogue stores
-    // SiLU(gate_j) * up_j as fp16 hi (+ lo) into act[token][N / 2] instead of the f32 rows
-    __half* act_hi; __half* act_lo;
-};
-
-__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
-    uint32_t r;
-    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
-    return r;
-}
-__device__ __forceinline__ __half2 as_h2(uint32_t v) { return *reinterpret_cast<__half2*>(&v); }
-__device__ __forceinline__ uint32_t as_u32(__half2 v) { return *reinterpret_cast<uint32_t*>(&v); }
-
-// two integer weights (exact in fp16) times the block scale: hi = rn16(q*d), lo = rn16(q*d - hi).  The fp16 multiply
-// rounds the exact product once and the fused multiply-add forms q*d - hi exactly before its one rounding, so
-// hi + lo carries the 19-bit product q*d to the last bit (|lo| <= ulp(hi)/2 is itself exact in fp16).
-__device__ __forceinline__ void scale_split(__half2 q, __half2 d, uint32_t& hi, uint32_t& lo) {
-    const __half2 h = __hmul2(q, d);
-    hi = as_u32(h);
-    lo = as_u32(__hfma2(q, d, __hneg2(h)));
-}
-
 // instruction descriptor: D f32, A/B f16, both K-major, M = 128 weight rows, N = NT tokens
 template <int NT> struct TsIdesc { static constexpr uint32_t value = (1u << 4) | (uint32_t(NT >> 3) << 17) | (uint32_t(128 >> 4) << 24); };
 
@@ -131,48 +106,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
           "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
           "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
         : "r"(taddr) : "memory");
-}
-
-// 32 consecutive weights of one row (one quantisation block) -> 16 + 16 packed fp16 pairs (hi, lo)
-template <int QUANT, bool SPLIT>
-__device__ __forceinline__ void dequant_block(const uint32_t* cur, __half2 d2, uint32_t (&hi)[16], uint32_t (&lo)[16]) {
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {      // 8 values per group
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {  // 2 values per register
-            __half2 q;
-            const uint32_t sel = (i & 1) ? 0x4342u : 0x4140u;
-            if (QUANT == FORGE_Q8_0) {
-                const uint32_t word = cur[2 * c + (i >> 1)];
-                q = __hsub2(as_h2(prmt(word ^ 0x80808080u, 0x64646464u, sel)), __float2half2_rn(1152.f));
-            } else {
-                const uint32_t word = cur[2 * (c & 1) + (i >> 1)];
-                const uint32_t two = prmt(word, 0u, sel) >> ((c >> 1) * 4);
-                q = __hsub2(as_h2((two & 0x000F000Fu) | 0x64006400u), __float2half2_rn(1032.f));
-            }
-            if (SPLIT) scale_split(q, d2, hi[4 * c + i], lo[4 * c + i]);
-            else hi[4 * c + i] = as_u32(__hmul2(q, d2));
-        }
-    }
-}
-
-// K-quant rows in the expanded row-major layout (FORGE_KQ_SOA): 32 int8 values and {s_lo, s_hi, mn}; the value
-// s * q - mn is formed in f32 (one fused rounding) and split into hi = rn16(w), lo = rn16(w - hi): 22 bits of w.
-template <bool SPLIT>
-__device__ __forceinline__ void dequant_block_kq(const uint32_t* cur, float4 sc, uint32_t (&hi)[16], uint32_t (&lo)[16]) {
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {  // register j = elements 2j, 2j + 1
-        const uint32_t word = cur[j >> 1];
-        const int q0 = int(int8_t(word >> (16 * (j & 1)))), q1 = int(int8_t(word >> (16 * (j & 1) + 8)));
-        const float s = j < 8 ? sc.x : sc.y;
-        const float w0 = fmaf(s, float(q0), -sc.z), w1 = fmaf(s, float(q1), -sc.z);
-        const __half2 h = __floats2half2_rn(w0, w1);
-        hi[j] = as_u32(h);
-        if (SPLIT) {
-            const float2 hf = __half22float2(h);
-            lo[j] = as_u32(__floats2half2_rn(w0 - hf.x, w1 - hf.y));
-        }
-    }
 }
 
 template <int QUANT, int NT, bool SPLIT, int XS>
@@ -786,7 +719,8 @@ bool gemm_tc5_supported(const QWeight& w) { return w.K % BK == 0 && w.K >= BK; }
 int gemm_tc5_ksplit(const QWeight& w) { return std::max(1, std::min(4, w.K / 1024)); }
 
 int32_t gemm_tc5(float* out, const __half* A, const __half* Alo, const QWeight& w, int m, const float* resid, int* err, cudaStream_t st,
-                 int ksplit, size_t part_stride, __half* act_hi, __half* act_lo) {
+                 int ksplit, size_t part_stride, __half* act_hi, __half* act_lo, int* parts) {
+    if (parts) *parts = ksplit;
     if (m <= 0) return FORGE_OK;
     if (!gemm_tc5_supported(w)) { set_error("tcgen05 gemm: K=%d must be a multiple of %d", w.K, BK); return FORGE_ERR_SHAPE; }
     if (ksplit < 1 || ksplit > w.K / BK || (ksplit > 1 && (resid || act_hi))) { set_error("tcgen05 gemm: bad K split"); return FORGE_ERR_INVALID_ARG; }
@@ -801,7 +735,12 @@ int32_t gemm_tc5(float* out, const __half* A, const __half* Alo, const QWeight& 
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    // Token tile: 128, 192 or 256.  A tile's cost is a fixed share (dequantising the 128 x K weight panel, prologue,
+    if (split && w.quant != FORGE_KQ_SOA) {
+        const PairPlan plan = gemm_pair_plan(w, m, ksplit, parts ? 0 : ksplit, sms);
+        if (parts) *parts = plan.parts;
+        return gemm_pair(out, A, Alo, w, m, resid, err, st, plan, ksplit, part_stride, act_hi, act_lo);
+    }
+    // single products and K-quant rows.  Token tile: 128, 192 or 256.  A tile's cost is a fixed share (dequantising the 128 x K weight panel, prologue,
     // epilogue) plus a share proportional to its tokens (measured on B200: 0.77 / 0.90 / 1.0 per CTA round); CTAs run
     // in whole rounds over the SMs.  Pick the cheapest.
     const long nt = (w.N + 127) / 128;
@@ -813,20 +752,18 @@ int32_t gemm_tc5(float* out, const __half* A, const __half* Alo, const QWeight& 
         const double cost = double((ctas + sms - 1) / sms) * (0.55 + 0.45 * cand / 256.0);
         if (cost < best_cost - 1e-9) { best_cost = cost; best = cand; }
     }
-#define FORGE_TS(Q)                                                                  \
-    do {                                                                             \
-        if (split) {                                                                 \
-            if (best == 256) return launch_ts<Q, 256, true>(A, Alo, p, st);          \
-            if (best == 192) return launch_ts<Q, 192, true>(A, Alo, p, st);          \
-            return launch_ts<Q, 128, true>(A, Alo, p, st);                           \
-        }                                                                            \
-        if (best == 256) return launch_ts<Q, 256, false>(A, Alo, p, st);             \
-        if (best == 192) return launch_ts<Q, 192, false>(A, Alo, p, st);             \
-        return launch_ts<Q, 128, false>(A, Alo, p, st);                              \
+#define FORGE_TS(Q, SPLIT)                                              \
+    do {                                                                \
+        if (best == 256) return launch_ts<Q, 256, SPLIT>(A, Alo, p, st); \
+        if (best == 192) return launch_ts<Q, 192, SPLIT>(A, Alo, p, st); \
+        return launch_ts<Q, 128, SPLIT>(A, Alo, p, st);                  \
     } while (0)
-    if (w.quant == FORGE_Q8_0) FORGE_TS(FORGE_Q8_0);
-    if (w.quant == FORGE_KQ_SOA) FORGE_TS(FORGE_KQ_SOA);
-    FORGE_TS(FORGE_Q4_0);
+    if (w.quant == FORGE_KQ_SOA) {
+        if (split) FORGE_TS(FORGE_KQ_SOA, true);
+        FORGE_TS(FORGE_KQ_SOA, false);
+    }
+    if (w.quant == FORGE_Q8_0) FORGE_TS(FORGE_Q8_0, false);
+    FORGE_TS(FORGE_Q4_0, false);
 #undef FORGE_TS
 }
 

@@ -223,8 +223,9 @@ int32_t row_sliced_gemm_norm(ForgeModel* m, const QWeight& w, const __half* a, c
     const int ks = gemm_tc5_ksplit(w);
     if (m->cfg.tp_world == 1 && ks > 1 && gemm_tc5_supported(w) && m->p_parts) {
         const size_t stride = size_t(n) * m->h;
-        FORGE_TRY(gemm_tc5(m->p_parts, a, alo, w, n, nullptr, m->d_err, st, ks, stride));
-        return add_parts_rms_norm_f16(m->p_hidden, m->p_parts, ks, stride, m->p_normed, nlo, next_norm, n, m->h, m->cfg.rms_norm_eps, st);
+        int parts;
+        FORGE_TRY(gemm_tc5(m->p_parts, a, alo, w, n, nullptr, m->d_err, st, ks, stride, nullptr, nullptr, &parts));
+        return add_parts_rms_norm_f16(m->p_hidden, m->p_parts, parts, stride, m->p_normed, nlo, next_norm, n, m->h, m->cfg.rms_norm_eps, st);
     }
     FORGE_TRY(row_sliced_gemm(m, w, a, alo, n, st));
     if (next_norm) FORGE_TRY(rms_norm_f16(m->p_normed, nlo, m->p_hidden, next_norm, n, m->h, m->cfg.rms_norm_eps, st));
@@ -285,7 +286,8 @@ int32_t prefill_seq(ForgeModel* m, ForgeKV* kv, int seq, const uint32_t* tokens_
         // memory, see gemm_tc5_ksplit) whose partials the epilogue kernel adds
         const int qks = (m->cfg.tp_world == 1 && gemm_tc5_supported(L.qkv) && m->p_qkv_parts) ? std::max(1, std::min(4, L.qkv.K / 1024)) : 1;
         const size_t qstride = size_t(n) * (m->qk + 2 * m->kv);
-        if (qks > 1) FORGE_TRY(gemm_tc5(m->p_qkv_parts, m->p_normed, nlo, L.qkv, n, nullptr, m->d_err, st, qks, qstride));
+        int qparts = 1;
+        if (qks > 1) FORGE_TRY(gemm_tc5(m->p_qkv_parts, m->p_normed, nlo, L.qkv, n, nullptr, m->d_err, st, qks, qstride, nullptr, nullptr, &qparts));
         else FORGE_TRY(gemm_f16a(m->p_qkv, m->p_normed, nlo, L.qkv, n, nullptr, m->d_err, st));
         const float* qkv_src = qks > 1 ? m->p_qkv_parts : m->p_qkv;
         // The attention runs in its precise form (queries and probabilities as fp16 hi + lo pairs, output to ~1e-6) whenever
@@ -293,7 +295,7 @@ int32_t prefill_seq(ForgeModel* m, ForgeKV* kv, int seq, const uint32_t* tokens_
         // compounds past the 1e-3 per-layer gate on 32-layer models.  K-quant models need it in any case (their attention
         // output is rounded to 8 bits in front of o_proj).
         const bool precise = m->any_kquant || m->gemm_passes == 3;
-        FORGE_TRY(qkv_post(qkv_src, n, base, L.qkv_bias, m->rope, m->p_q16, precise ? m->p_q16_lo : nullptr, kp, vp, page_row, m->qk, m->kv, m->hd, st, qks, qstride));
+        FORGE_TRY(qkv_post(qkv_src, n, base, L.qkv_bias, m->rope, m->p_q16, precise ? m->p_q16_lo : nullptr, kp, vp, page_row, m->qk, m->kv, m->hd, st, qparts, qstride));
         AttnPrefillArgs pa{m->p_attn16, alo, nullptr, m->p_q16, kp, vp, page_row, n, base, m->nq, m->nkv, m->hd, c.sliding_window};
         if (precise) { pa.q16_lo = m->p_q16_lo; pa.precise = 1; }
         pa.pool_rows = size_t(kv->num_pages) * FORGE_KV_PAGE; pa.err = m->d_err;
@@ -453,10 +455,11 @@ int32_t decode_launches_gemm(ForgeModel* m, ForgeKV* kv, int batch, bool greedy,
         // q/k/v as K slices like the prompt's (more CTAs for a product of few row tiles; the epilogue adds the slices)
         const int qks = (c.tp_world == 1 && split && gemm_tc5_supported(L.qkv) && m->p_qkv_parts) ? std::max(1, std::min(4, L.qkv.K / 1024)) : 1;
         const size_t qstride = size_t(n) * (m->qk + 2 * m->kv);
-        if (qks > 1) FORGE_TRY(gemm_tc5(m->p_qkv_parts, m->p_normed, nlo, L.qkv, n, nullptr, m->d_err, st, qks, qstride));
+        int qparts = 1;
+        if (qks > 1) FORGE_TRY(gemm_tc5(m->p_qkv_parts, m->p_normed, nlo, L.qkv, n, nullptr, m->d_err, st, qks, qstride, nullptr, nullptr, &qparts));
         else FORGE_TRY(gemm_f16a(m->p_qkv, m->p_normed, nlo, L.qkv, n, nullptr, m->d_err, st));
         FORGE_TRY(qkv_post_rows(qks > 1 ? m->p_qkv_parts : m->p_qkv, n, L.qkv_bias, m->rope, m->d_q, kp, vp, kv->d_page_table, kv->d_seq_len,
-                                kv->pages_per_seq, m->qk, m->kv, m->hd, st, qks, qstride));
+                                kv->pages_per_seq, m->qk, m->kv, m->hd, st, qparts, qstride));
         AttnDecodeArgs da{m->d_attn, m->d_q, kp, vp, kv->d_page_table, kv->pages_per_seq, kv->d_seq_len, 0,
                           n, m->nq, m->nkv, m->hd, kv->max_seq, kv->attn_ws, kv->attn_counters, kv->splits[n], c.sliding_window};
         da.map_k = kv->k_map; da.map_v = kv->v_map; da.row_base = int(size_t(l) * kv->num_pages * FORGE_KV_PAGE); da.err = m->d_err; da.f32 = m->any_kquant;

@@ -43,6 +43,29 @@ def test_prompt_product_edges(oracle, quant, m, K, N):
     lib.forge_packed_destroy(pk)
 
 
+@pytest.mark.parametrize("quant,hidden,ffn,n", [(4, 2048, 4096, 33), (8, 2048, 5120, 200), (4, 3072, 2048, 65), (8, 1024, 8192, 449)])
+def test_prompt_slices(oracle, quant, hidden, ffn, n):
+    """K slices of products, added up by the pair that owns the tile or left as partial outputs, ragged last tiles, the SiLU epilogue.  The bound is eight products
+    of 3e-5 each and twice what rounding K and V to fp16 makes of a difference of 6e-6 (sqrt(6e-6 * 2^-11))."""
+    from forge_llm_b200 import configs, runtime, synth
+    c = configs.tiny(quant, hd=64, nq=hidden // 64, nkv=hidden // 128, layers=2, hidden=hidden, ffn=ffn, vocab=1000)
+    blob = synth.make_weights_bin(c)
+    gm = runtime.Model(c, blob)
+    om = oracle.OracleModel(c, blob, kv_mode=oracle.KV_F16)
+    p = synth.prompt_tokens(c, n, seed=n)
+    want = om.forward_prefill(p)
+    kv = gm.new_cache(max_seq=n + 2, batch=1)
+    first = None
+    for _ in range(5):
+        kv.reset()
+        got = gm.forward_prefill(p, kv)
+        assert rel_l2(got, want) < 3.5e-4
+        first = got if first is None else first
+        assert np.array_equal(got, first)
+    kv.close()
+    gm.close()
+
+
 @pytest.mark.parametrize("hd,nq,nkv", [(64, 16, 1), (64, 18, 2), (96, 9, 1), (128, 7, 7), (128, 16, 2)])
 @pytest.mark.parametrize("seq", [1, 15, 16, 17, 63, 65, 511, 513, 8300])
 def test_decode_attention_edges(oracle, hd, nq, nkv, seq):
