@@ -185,6 +185,8 @@ __global__ void __launch_bounds__(kThreads) attn_prefill_tc5_kernel(const __grid
     if (warp == 0) {
         // ---------------- TMA producer: the query tile once, then the K and V pages of every key tile
         if (lane == 0) {
+            pdl_wait();      // queries, keys, values and the page table; what the other warps write follows from these
+            pdl_trigger();
             mbar_expect_tx(&q_full, uint32_t(Q_BYTES));
             for (int c = 0; c < NCH; ++c) {
                 tma_load_3d(sQ + c * Q_CHUNK, &map_q, c * 64, h, q0, &q_full);
@@ -410,7 +412,7 @@ int32_t launch(const CUtensorMap& mq, const CUtensorMap& mql, const CUtensorMap&
     auto kern = attn_prefill_tc5_kernel<HD, SW, PRECISE>;
     FORGE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     dim3 grid((p.a.m + BM - 1) / BM, p.a.nq);
-    kern<<<grid, kThreads, smem, st>>>(mq, mql, mk, mv, p);
+    FORGE_CUDA(launch_pdl(kern, grid, dim3(kThreads), smem, st, mq, mql, mk, mv, p));
     FORGE_LAUNCH_CHECK();
     return FORGE_OK;
 }

@@ -29,9 +29,13 @@ __device__ __forceinline__ void store_split(__half* hi, __half* lo, size_t i, fl
     if (lo) lo[i] = __float2half_rn(v - __half2float(h));
 }
 
+// Kernels of a chain wait first for the one in front (their pointers are not restrict: a load of what another kernel writes must not move in front of the wait) and only
+// then let the next be scheduled, so that whatever starts early finds everything but its direct predecessor complete.
 template <typename OutT>
-__global__ void rms_norm_kernel(OutT* __restrict__ out, __half* __restrict__ lo, const float* __restrict__ in, const float* __restrict__ w, int n, float eps) {
+__global__ void rms_norm_kernel(OutT* out, __half* lo, const float* in, const float* w, int n, float eps) {
     __shared__ float red[32];
+    pdl_wait();
+    pdl_trigger();
     const float* x = in + size_t(blockIdx.x) * n;
     float ss = 0.f;
     for (int i = threadIdx.x; i < n; i += blockDim.x) { float v = x[i]; ss += v * v; }
@@ -47,9 +51,10 @@ __global__ void rms_norm_kernel(OutT* __restrict__ out, __half* __restrict__ lo,
 // fp16 hi/lo output for rows of at most 256 * 4 * NV floats: the row is read once with 128-bit loads and stays in
 // registers between the sum of squares and the scaling
 template <int NV>
-__global__ void __launch_bounds__(256) rms_norm_f16_vec_kernel(__half* __restrict__ out, __half* __restrict__ lo, const float* __restrict__ in,
-                                                                const float* __restrict__ w, int n, float eps) {
+__global__ void __launch_bounds__(256) rms_norm_f16_vec_kernel(__half* out, __half* lo, const float* in, const float* w, int n, float eps) {
     __shared__ float red[32];
+    pdl_wait();
+    pdl_trigger();
     const float* x = in + size_t(blockIdx.x) * n;
     float4 v[NV];
     float ss = 0.f;
@@ -81,9 +86,10 @@ __global__ void __launch_bounds__(256) rms_norm_f16_vec_kernel(__half* __restric
 // residual_add (emit.rs:455-459) of a product that arrives as K-slice partials, fused with the rms_norm (emit.rs:327-334)
 // of the next operator: hidden += part_0 + part_1 + ... in slice order, the row stays in registers for the normalisation
 template <int NV>
-__global__ void __launch_bounds__(256) add_parts_norm_kernel(float* __restrict__ hidden, const float* __restrict__ parts, int nparts, size_t pstride,
-                                                              __half* __restrict__ out, __half* __restrict__ lo, const float* __restrict__ w, int n, float eps) {
+__global__ void __launch_bounds__(256) add_parts_norm_kernel(float* hidden, const float* parts, int nparts, size_t pstride, __half* out, __half* lo, const float* w, int n, float eps) {
     __shared__ float red[32];
+    pdl_wait();
+    pdl_trigger();
     float* x = hidden + size_t(blockIdx.x) * n;
     const float* pr = parts + size_t(blockIdx.x) * n;
     float4 v[NV];
@@ -126,7 +132,9 @@ __global__ void __launch_bounds__(256) add_parts_norm_kernel(float* __restrict__
 }
 
 // thread per (row, head, pair): adjacent-pair rotation, table = {cos, sin}[pos][hd/2]
-__global__ void rope_kernel(float* data, int rows, int base_pos, int hd, int heads, const float2* __restrict__ table) {
+__global__ void rope_kernel(float* data, int rows, int base_pos, int hd, int heads, const float2* table) {
+    pdl_wait();
+    pdl_trigger();
     int half = hd / 2;
     long total = long(rows) * heads * half;
     for (long i = blockIdx.x * long(blockDim.x) + threadIdx.x; i < total; i += long(gridDim.x) * blockDim.x) {
@@ -141,6 +149,8 @@ __global__ void rope_kernel(float* data, int rows, int base_pos, int hd, int hea
 }
 
 __global__ void silu_mul_kernel(float* out, const float* g, const float* u, size_t n) {
+    pdl_wait();
+    pdl_trigger();
     for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
         float x = g[i];
         out[i] = (x / (1.0f + expf(-x))) * u[i];
@@ -156,6 +166,8 @@ __global__ void silu_mul_f16_kernel(__half* out, __half* lo, const float2* gu, s
 }
 
 __global__ void residual_add_kernel(float* a, const float* b, size_t n) {
+    pdl_wait();
+    pdl_trigger();
     for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) a[i] += b[i];
 }
 
@@ -243,7 +255,9 @@ __global__ void gather_act_kernel(uint4* dst, const uint4* src, const int32_t* i
     for (int i = threadIdx.x; i < n16; i += blockDim.x) dst[size_t(blockIdx.x) * n16 + i] = src[size_t(idx[blockIdx.x]) * ld16 + i];
 }
 
+// (a reader of the cache may take rows in front of its wait, so this one lets nothing start early)
 __global__ void kv_append_contig_kernel(__half* kc, __half* vc, const float* k, const float* v, size_t n, size_t off) {
+    pdl_wait();
     for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
         kc[off + i] = __float2half_rn(k[i]);
         vc[off + i] = __float2half_rn(v[i]);
@@ -252,9 +266,10 @@ __global__ void kv_append_contig_kernel(__half* kc, __half* vc, const float* k, 
 
 // prefill glue: fused [q;k;v] f32 rows -> (+bias) -> RoPE on q,k -> q fp16, k/v into the paged cache
 // (the product may arrive as `nparts` K-slice partials, pstride floats apart: they are added in slice order)
-__global__ void qkv_post_kernel(const float* __restrict__ qkv, int nparts, size_t pstride, int m, int base_pos, const float* __restrict__ bias,
-                                const float2* __restrict__ rope, __half* __restrict__ q16, __half* __restrict__ q16_lo, __half* __restrict__ k_pool,
-                                __half* __restrict__ v_pool, const int32_t* __restrict__ page_row, int qk, int kv, int hd) {
+__global__ void qkv_post_kernel(const float* qkv, int nparts, size_t pstride, int m, int base_pos, const float* __restrict__ bias, const float2* __restrict__ rope, __half* q16,
+                                __half* q16_lo, __half* k_pool, __half* v_pool, const int32_t* page_row, int qk, int kv, int hd) {
+    pdl_wait();
+    pdl_trigger();
     const int npairs = (qk + 2 * kv) / 2;
     const int r = blockIdx.x;
     const int pos = base_pos + r;
@@ -289,10 +304,10 @@ __global__ void qkv_post_kernel(const float* __restrict__ qkv, int nparts, size_
 
 // batched decode glue: row b of the fused [q;k;v] product belongs to sequence b at position seq_len[b]:
 // (+bias) -> RoPE on q,k -> q f32 [b][qk], k/v into that sequence's cache page
-__global__ void qkv_post_rows_kernel(const float* __restrict__ qkv, int nparts, size_t pstride, const float* __restrict__ bias, const float2* __restrict__ rope,
-                                     float* __restrict__ q_out, __half* __restrict__ k_pool, __half* __restrict__ v_pool,
-                                     const int32_t* __restrict__ page_table, const int32_t* __restrict__ seq_len, int pages_per_seq,
-                                     int qk, int kv, int hd) {
+__global__ void qkv_post_rows_kernel(const float* qkv, int nparts, size_t pstride, const float* __restrict__ bias, const float2* __restrict__ rope, float* q_out, __half* k_pool,
+                                     __half* v_pool, const int32_t* page_table, const int32_t* seq_len, int pages_per_seq, int qk, int kv, int hd) {
+    pdl_wait();
+    pdl_trigger();
     const int npairs = (qk + 2 * kv) / 2;
     const int b = blockIdx.x;
     const int pos = seq_len[b];
@@ -418,6 +433,8 @@ __global__ void argmax_slices_kernel(uint32_t* result, const float* logits, int 
 }
 
 __global__ void f32_to_f16_kernel(__half* out, __half* lo, const float* in, size_t n) {
+    pdl_wait();
+    pdl_trigger();
     for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) store_split(out, lo, i, in[i]);
 }
 
@@ -472,16 +489,16 @@ inline int grid_for(size_t n, int threads = 256) {
 
 int32_t rms_norm_f32(float* out, const float* in, const float* w, int rows, int n, float eps, cudaStream_t st) {
     if (rows <= 0) return FORGE_OK;
-    rms_norm_kernel<float><<<rows, 256, 0, st>>>(out, nullptr, in, w, n, eps);
+    FORGE_CUDA(launch_pdl(rms_norm_kernel<float>, dim3(rows), dim3(256), 0, st, out, nullptr, in, w, n, eps));
     FORGE_LAUNCH_CHECK();
     return FORGE_OK;
 }
 int32_t rms_norm_f16(__half* out, __half* lo, const float* in, const float* w, int rows, int n, float eps, cudaStream_t st) {
     if (rows <= 0) return FORGE_OK;
-    if (n % 4 == 0 && n <= 2048) rms_norm_f16_vec_kernel<2><<<rows, 256, 0, st>>>(out, lo, in, w, n, eps);
-    else if (n % 4 == 0 && n <= 4096) rms_norm_f16_vec_kernel<4><<<rows, 256, 0, st>>>(out, lo, in, w, n, eps);
-    else if (n % 4 == 0 && n <= 8192) rms_norm_f16_vec_kernel<8><<<rows, 256, 0, st>>>(out, lo, in, w, n, eps);
-    else rms_norm_kernel<__half><<<rows, 256, 0, st>>>(out, lo, in, w, n, eps);
+    if (n % 4 == 0 && n <= 2048) FORGE_CUDA(launch_pdl(rms_norm_f16_vec_kernel<2>, dim3(rows), dim3(256), 0, st, out, lo, in, w, n, eps));
+    else if (n % 4 == 0 && n <= 4096) FORGE_CUDA(launch_pdl(rms_norm_f16_vec_kernel<4>, dim3(rows), dim3(256), 0, st, out, lo, in, w, n, eps));
+    else if (n % 4 == 0 && n <= 8192) FORGE_CUDA(launch_pdl(rms_norm_f16_vec_kernel<8>, dim3(rows), dim3(256), 0, st, out, lo, in, w, n, eps));
+    else FORGE_CUDA(launch_pdl(rms_norm_kernel<__half>, dim3(rows), dim3(256), 0, st, out, lo, in, w, n, eps));
     FORGE_LAUNCH_CHECK();
     return FORGE_OK;
 }
@@ -489,22 +506,22 @@ int32_t add_parts_rms_norm_f16(float* hidden, const float* parts, int nparts, si
                                int rows, int n, float eps, cudaStream_t st) {
     if (rows <= 0) return FORGE_OK;
     if (n % 4 || n > 8192 || nparts < 1 || nparts > 4) { set_error("add_parts_rms_norm: row length %d / %d slices unsupported", n, nparts); return FORGE_ERR_SHAPE; }
-    if (n <= 2048) add_parts_norm_kernel<2><<<rows, 256, 0, st>>>(hidden, parts, nparts, pstride, out, lo, w, n, eps);
-    else if (n <= 4096) add_parts_norm_kernel<4><<<rows, 256, 0, st>>>(hidden, parts, nparts, pstride, out, lo, w, n, eps);
-    else add_parts_norm_kernel<8><<<rows, 256, 0, st>>>(hidden, parts, nparts, pstride, out, lo, w, n, eps);
+    if (n <= 2048) FORGE_CUDA(launch_pdl(add_parts_norm_kernel<2>, dim3(rows), dim3(256), 0, st, hidden, parts, nparts, pstride, out, lo, w, n, eps));
+    else if (n <= 4096) FORGE_CUDA(launch_pdl(add_parts_norm_kernel<4>, dim3(rows), dim3(256), 0, st, hidden, parts, nparts, pstride, out, lo, w, n, eps));
+    else FORGE_CUDA(launch_pdl(add_parts_norm_kernel<8>, dim3(rows), dim3(256), 0, st, hidden, parts, nparts, pstride, out, lo, w, n, eps));
     FORGE_LAUNCH_CHECK();
     return FORGE_OK;
 }
 int32_t rope_rows(float* data, int rows, int base_pos, int head_dim, int heads, const float* table, cudaStream_t st) {
     size_t n = size_t(rows) * heads * (head_dim / 2);
     if (n == 0) return FORGE_OK;
-    rope_kernel<<<grid_for(n), 256, 0, st>>>(data, rows, base_pos, head_dim, heads, reinterpret_cast<const float2*>(table));
+    FORGE_CUDA(launch_pdl(rope_kernel, dim3(grid_for(n)), dim3(256), 0, st, data, rows, base_pos, head_dim, heads, reinterpret_cast<const float2*>(table)));
     FORGE_LAUNCH_CHECK();
     return FORGE_OK;
 }
 int32_t silu_mul_f32(float* out, const float* g, const float* u, size_t n, cudaStream_t st) {
     if (n == 0) return FORGE_OK;
-    silu_mul_kernel<<<grid_for(n), 256, 0, st>>>(out, g, u, n);
+    FORGE_CUDA(launch_pdl(silu_mul_kernel, dim3(grid_for(n)), dim3(256), 0, st, out, g, u, n));
     FORGE_LAUNCH_CHECK();
     return FORGE_OK;
 }
@@ -517,7 +534,7 @@ int32_t silu_mul_f16(__half* out, __half* lo, const float* gu, int rows, int ffn
 }
 int32_t residual_add_f32(float* a, const float* b, size_t n, cudaStream_t st) {
     if (n == 0) return FORGE_OK;
-    residual_add_kernel<<<grid_for(n), 256, 0, st>>>(a, b, n);
+    FORGE_CUDA(launch_pdl(residual_add_kernel, dim3(grid_for(n)), dim3(256), 0, st, a, b, n));
     FORGE_LAUNCH_CHECK();
     return FORGE_OK;
 }
@@ -530,14 +547,15 @@ int32_t embedding_rows(float* out, const float* table, const uint32_t* tokens, i
 int32_t kv_append_contig(__half* kc, __half* vc, const float* k, const float* v, int rows, int base_pos, int kvd, cudaStream_t st) {
     size_t n = size_t(rows) * kvd;
     if (n == 0) return FORGE_OK;
-    kv_append_contig_kernel<<<grid_for(n), 256, 0, st>>>(kc, vc, k, v, n, size_t(base_pos) * kvd);
+    FORGE_CUDA(launch_pdl(kv_append_contig_kernel, dim3(grid_for(n)), dim3(256), 0, st, kc, vc, k, v, n, size_t(base_pos) * kvd));
     FORGE_LAUNCH_CHECK();
     return FORGE_OK;
 }
 int32_t qkv_post(const float* qkv, int m, int base_pos, const float* bias, const float* rope, __half* q16, __half* q16_lo,
                  __half* k_pool, __half* v_pool, const int32_t* page_row, int qk, int kv, int hd, cudaStream_t st, int nparts, size_t pstride) {
     if (m <= 0) return FORGE_OK;
-    qkv_post_kernel<<<m, 256, 0, st>>>(qkv, nparts, pstride, m, base_pos, bias, reinterpret_cast<const float2*>(rope), q16, q16_lo, k_pool, v_pool, page_row, qk, kv, hd);
+    FORGE_CUDA(launch_pdl(qkv_post_kernel, dim3(m), dim3(256), 0, st, qkv, nparts, pstride, m, base_pos, bias, reinterpret_cast<const float2*>(rope), q16, q16_lo, k_pool, v_pool,
+                          page_row, qk, kv, hd));
     FORGE_LAUNCH_CHECK();
     return FORGE_OK;
 }
@@ -547,8 +565,8 @@ int32_t qkv_post_rows(const float* qkv, int batch, const float* bias, const floa
     if (batch <= 0) return FORGE_OK;
     const int npairs = (qk + 2 * kv) / 2;
     if (nparts < 1 || nparts > 4) { set_error("qkv_post_rows: %d slices unsupported", nparts); return FORGE_ERR_INVALID_ARG; }
-    qkv_post_rows_kernel<<<dim3(batch, (npairs + 255) / 256), 256, 0, st>>>(qkv, nparts, pstride, bias, reinterpret_cast<const float2*>(rope), q_out, k_pool, v_pool, page_table, seq_len,
-                                                pages_per_seq, qk, kv, hd);
+    FORGE_CUDA(launch_pdl(qkv_post_rows_kernel, dim3(batch, (npairs + 255) / 256), dim3(256), 0, st, qkv, nparts, pstride, bias, reinterpret_cast<const float2*>(rope), q_out, k_pool,
+                          v_pool, page_table, seq_len, pages_per_seq, qk, kv, hd));
     FORGE_LAUNCH_CHECK();
     return FORGE_OK;
 }
@@ -611,7 +629,7 @@ int32_t q8_round_f16(__half* hi, __half* lo, size_t n, cudaStream_t st) {
 
 int32_t f32_to_f16(__half* out, __half* lo, const float* in, size_t n, cudaStream_t st) {
     if (n == 0) return FORGE_OK;
-    f32_to_f16_kernel<<<grid_for(n), 256, 0, st>>>(out, lo, in, n);
+    FORGE_CUDA(launch_pdl(f32_to_f16_kernel, dim3(grid_for(n)), dim3(256), 0, st, out, lo, in, n));
     FORGE_LAUNCH_CHECK();
     return FORGE_OK;
 }

@@ -196,6 +196,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) gem
         // ---------------- activations
         if (lane == 0) {
             pdl_wait();
+            pdl_trigger();
             bool ok = true;
             int st = 0;
             uint32_t use = 0;
@@ -427,7 +428,7 @@ int32_t launch_pair(const __half* A, const __half* Alo, PairParams p, int pairs,
         if (p.bulk) FORGE_TRY(out_map(&mo, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, t.out, t.N, t.m, p.parts, size_t(t.N) * 4, part, 128));
     }
     FORGE_CUDA(cudaFuncSetAttribute(gemm_pair_kernel<QUANT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem));
-    gemm_pair_kernel<QUANT><<<2 * pairs, kPairThreads, kPairSmem, st>>>(mh, ml, mw, mo, mol, p);
+    FORGE_CUDA(launch_pdl(gemm_pair_kernel<QUANT>, dim3(2 * pairs), dim3(kPairThreads), kPairSmem, st, mh, ml, mw, mo, mol, p));
     FORGE_LAUNCH_CHECK();
     return FORGE_OK;
 }

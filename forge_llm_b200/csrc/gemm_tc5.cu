@@ -440,6 +440,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1) gemm_small_kernel(const __gr
     } else if (warp == 0) {
         // ---------------- TMA producer: per group, the rows' hi and lo tiles of its K steps (columns past K read as zero)
         if (lane == 0) {
+            pdl_wait();      // the rows; weights and scales are constant, and what the epilogue reads and writes follows from the rows
+            pdl_trigger();
             for (int gi = 0; gi < ng; ++gi) {
                 const int s = gi % XS, use = gi / XS;
                 if (use > 0 && !mbar_wait(&empty_x[s], (use - 1) & 1, &s_err)) { atomicExch(&s_err, 1); break; }
@@ -703,7 +705,7 @@ int32_t launch_small(const __half* A, const __half* Alo, const Tc5Params& p, cud
     auto kern = gemm_small_kernel<QUANT, NT>;
     FORGE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     dim3 grid((p.N + 127) / 128, 1, p.ksplit);
-    kern<<<grid, kSmallThreads, smem, st>>>(mh, ml, mw, p);
+    FORGE_CUDA(launch_pdl(kern, grid, dim3(kSmallThreads), smem, st, mh, ml, mw, p));
     FORGE_LAUNCH_CHECK();
     return FORGE_OK;
 }

@@ -99,29 +99,40 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_batch_kernel(BatchParams p) 
         // ---- producer lane: for every unit of this CTA, the stages of its K slice: weights (one copy in the 128-row
         // layout, one per row tile in the 16-row layout) and the packed activations of the same k-blocks
         if (lane == 0) {
-            int cc = 0;
-            for (int u = blockIdx.x; u < p.units; u += gridDim.x) {
-                const int grp = u / p.slices, slice = u - grp * p.slices;
-                int c0, c1;
-                slice_range(chunks, p.slices, slice, c0, c1);
-                for (int c = c0; c < c1; ++c, ++cc) {
-                    const int st = cc % STAGES, use = cc / STAGES;
-                    if (use > 0 && !mbar_wait(&sh.empty_bar[st], (use - 1) & 1, &sh.err)) { atomicExch(&sh.err, 1); return; }
-                    if (*reinterpret_cast<volatile int*>(&sh.err)) return;
-                    const int kb0 = c * CKB, nkb = min(CKB, p.kb - kb0);
-                    unsigned char* dst = smem + size_t(st) * STAGE;
-                    const int tiles = wide ? kBandTiles : min(kBandTiles, p.bands16 - grp * kBandTiles);   // row tiles of the group that exist
-                    const uint32_t wbytes = uint32_t(nkb) * tiles * T::BYTES, abytes = uint32_t(nkb) * 2 * NCG * 256;
-                    mbar_expect_tx(&sh.full_bar[st], wbytes + abytes);
-                    if (wide) {
-                        bulk_g2s(dst, p.w + (size_t(grp) * p.kb + kb0) * kBandTiles * T::BYTES, wbytes, &sh.full_bar[st]);
-                    } else {
+            // weights are constant: those of the first stages are requested in front of the wait for the kernel that packs the activations
+            for (int early = 1; early >= 0; --early) {
+                int cc = 0;
+                bool room = true;
+                for (int u = blockIdx.x; u < p.units && room; u += gridDim.x) {
+                    const int grp = u / p.slices, slice = u - grp * p.slices;
+                    int c0, c1;
+                    slice_range(chunks, p.slices, slice, c0, c1);
+                    for (int c = c0; c < c1; ++c, ++cc) {
+                        const int st = cc % STAGES, use = cc / STAGES;
+                        if (early && use > 0) { room = false; break; }
+                        if (use > 0 && !mbar_wait(&sh.empty_bar[st], (use - 1) & 1, &sh.err)) { atomicExch(&sh.err, 1); return; }
+                        if (*reinterpret_cast<volatile int*>(&sh.err)) return;
+                        const int kb0 = c * CKB, nkb = min(CKB, p.kb - kb0);
+                        unsigned char* dst = smem + size_t(st) * STAGE;
+                        const int tiles = wide ? kBandTiles : min(kBandTiles, p.bands16 - grp * kBandTiles);   // row tiles of the group that exist
+                        const uint32_t wbytes = uint32_t(nkb) * tiles * T::BYTES, abytes = uint32_t(nkb) * 2 * NCG * 256;
+                        if (early || use > 0) {
+                            mbar_expect_tx(&sh.full_bar[st], wbytes + abytes);
+                            if (wide) {
+                                bulk_g2s(dst, p.w + (size_t(grp) * p.kb + kb0) * kBandTiles * T::BYTES, wbytes, &sh.full_bar[st]);
+                            } else {
 #pragma unroll 1
-                        for (int r8 = 0; r8 < tiles; ++r8)   // row tile r8 of the group is band grp * 8 + r8 of the 16-row layout
-                            bulk_g2s(dst + size_t(r8) * CKB * T::BYTES, p.w + (size_t(grp * kBandTiles + r8) * p.kb + kb0) * T::BYTES,
-                                     uint32_t(nkb) * T::BYTES, &sh.full_bar[st]);
+                                for (int r8 = 0; r8 < tiles; ++r8)   // row tile r8 of the group is band grp * 8 + r8 of the 16-row layout
+                                    bulk_g2s(dst + size_t(r8) * CKB * T::BYTES, p.w + (size_t(grp * kBandTiles + r8) * p.kb + kb0) * T::BYTES,
+                                             uint32_t(nkb) * T::BYTES, &sh.full_bar[st]);
+                            }
+                        }
+                        if (!early) bulk_g2s(dst + B::W_BYTES, p.act + size_t(kb0) * 2 * NCG * 32, abytes, &sh.full_bar[st]);
                     }
-                    bulk_g2s(dst + B::W_BYTES, p.act + size_t(kb0) * 2 * NCG * 32, abytes, &sh.full_bar[st]);
+                }
+                if (early) {
+                    pdl_wait();
+                    pdl_trigger();
                 }
             }
         }
@@ -273,8 +284,10 @@ enum PackMode { PACK_PLAIN = 0, PACK_NORM = 1, PACK_SILU = 2 };
 
 template <int QUANT>
 __global__ void __launch_bounds__(256) act_pack_kernel(float* x, size_t x_stride, const float* __restrict__ norm_w, float eps,
-                                                       int mode, int K, int ncg, uint2* __restrict__ dst, BatchTp tp) {
+                                                       int mode, int K, int ncg, uint2* dst, BatchTp tp) {
     __shared__ float s_red[8];
+    pdl_wait();
+    pdl_trigger();
     const int b = blockIdx.x;
     float* row = x + size_t(b) * x_stride;
     float inv = 1.0f;
@@ -343,7 +356,7 @@ int32_t launch_batch(const BatchParams& p, int grid, cudaStream_t st) {
     const size_t smem = size_t(B::STAGES) * B::STAGE;
     auto kern = gemv_batch_kernel<QUANT, NCG>;
     FORGE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    kern<<<grid, kThreads, smem, st>>>(p);
+    FORGE_CUDA(launch_pdl(kern, dim3(grid), dim3(kThreads), smem, st, p));
     FORGE_LAUNCH_CHECK();
     return FORGE_OK;
 }
@@ -381,8 +394,8 @@ int32_t gemv_batch_pack(uint2* dst, float* x, size_t x_stride, int nb, int K, in
     const int ncg = gemv_batch_ncg(nb);
     if (consume && (mode != PACK_NORM || !consume->local_ll || size_t(nb) * K > consume->cap)) { set_error("batched product: bad tensor-parallel consume"); return FORGE_ERR_INVALID_ARG; }
     const BatchTp tp = consume ? *consume : BatchTp();
-    if (quant == FORGE_Q8_0) act_pack_kernel<FORGE_Q8_0><<<nb, 256, 0, st>>>(x, x_stride, norm_w, eps, mode, K, ncg, dst, tp);
-    else act_pack_kernel<FORGE_Q4_0><<<nb, 256, 0, st>>>(x, x_stride, norm_w, eps, mode, K, ncg, dst, tp);
+    if (quant == FORGE_Q8_0) FORGE_CUDA(launch_pdl(act_pack_kernel<FORGE_Q8_0>, dim3(nb), dim3(256), 0, st, x, x_stride, norm_w, eps, mode, K, ncg, dst, tp));
+    else FORGE_CUDA(launch_pdl(act_pack_kernel<FORGE_Q4_0>, dim3(nb), dim3(256), 0, st, x, x_stride, norm_w, eps, mode, K, ncg, dst, tp));
     FORGE_LAUNCH_CHECK();
     return FORGE_OK;
 }

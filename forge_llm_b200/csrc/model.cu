@@ -221,7 +221,7 @@ int32_t row_sliced_gemm(ForgeModel* m, const QWeight& w, const __half* a, const 
 // and more CTAs for these few-row-tile matrices.
 int32_t row_sliced_gemm_norm(ForgeModel* m, const QWeight& w, const __half* a, const __half* alo, int n, const float* next_norm, __half* nlo, cudaStream_t st) {
     const int ks = gemm_tc5_ksplit(w);
-    if (m->cfg.tp_world == 1 && ks > 1 && gemm_tc5_supported(w) && m->p_parts) {
+    if (m->cfg.tp_world == 1 && gemm_tc5_supported(w) && m->p_parts) {
         const size_t stride = size_t(n) * m->h;
         int parts;
         FORGE_TRY(gemm_tc5(m->p_parts, a, alo, w, n, nullptr, m->d_err, st, ks, stride, nullptr, nullptr, &parts));

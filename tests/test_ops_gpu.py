@@ -354,3 +354,67 @@ def test_first_scratch_of_a_process_under_capture():
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     done = subprocess.run([sys.executable, "-c", CAPTURE], cwd=root, capture_output=True, text=True, timeout=300)
     assert done.returncode == 0, done.stderr[-2000:]
+
+
+@pytest.mark.parametrize("rows", [1, 9, 40])
+def test_operators_in_a_row_see_each_other(L, rows):
+    """Operators start while the one in front is still ending: a chain of them without waiting gives the bits of one that is waited for call by call, also where the buffers
+    and the library's scratch are used again at once."""
+    import torch
+    from forge_llm_b200 import synth
+    lib, check = L
+    hd, nq, nkv, h, ff, base = 64, 6, 2, 384, 1024, 70
+    rng = np.random.default_rng(rows)
+    packed = {}
+    for name, n, k in (("q", nq * hd, h), ("k", nkv * hd, h), ("v", nkv * hd, h), ("o", h, nq * hd), ("gate", ff, h), ("up", ff, h), ("down", h, ff)):
+        packed[name] = C.c_void_p()
+        w = dev(synth.quantize(8, rng.standard_normal((n, k), dtype=np.float32) * 0.05))
+        check(lib.forge_packed_create(8, w.data_ptr(), k, n, None, C.byref(packed[name])))
+    table = np.empty((base + 30 * rows + rows, hd // 2, 2), np.float32)
+    check(lib.forge_rope_table(table.ctypes.data, table.shape[0], hd, 10000.0))
+    table = dev(table)
+    x0, norm = dev(rng.standard_normal((rows, h), dtype=np.float32)), dev(1 + 0.1 * rng.standard_normal(h, dtype=np.float32))
+    kv0 = dev(rng.standard_normal((2, table.shape[0], nkv * hd), dtype=np.float32).astype(np.float16).view(np.uint16))
+
+    def layers(sync):
+        x, kv = x0.clone(), kv0.clone()
+        t = {n: torch.empty(rows, c, device="cuda") for n, c in (("y", h), ("q", nq * hd), ("k", nkv * hd), ("v", nkv * hd), ("a", nq * hd), ("g", ff), ("u", ff), ("p", h))}
+        p = {n: b.data_ptr() for n, b in t.items()}
+        torch.cuda.synchronize()
+
+        def call(fn, *a):
+            check(fn(*a, None))
+            if sync:
+                torch.cuda.synchronize()
+
+        pos = base
+        for _ in range(12):
+            call(lib.forge_rms_norm, p["y"], x.data_ptr(), norm.data_ptr(), rows, h, 1e-5)
+            for n in "qkv":
+                call(lib.forge_matmul_mat_packed, p[n], rows, p["y"], packed[n])
+            call(lib.forge_rope, p["q"], rows, pos, hd, nq, table.data_ptr())
+            call(lib.forge_rope, p["k"], rows, pos, hd, nkv, table.data_ptr())
+            call(lib.forge_kv_append_f16, kv[0].data_ptr(), kv[1].data_ptr(), p["k"], p["v"], rows, pos, nkv * hd)
+            if rows == 1:
+                call(lib.forge_attention_flash, p["a"], p["q"], kv[0].data_ptr(), kv[1].data_ptr(), pos + 1, nq, nkv, hd)
+            else:   # the last row alone: the decode attention right behind an append of several rows
+                t["a"].zero_()
+                call(lib.forge_attention_flash, p["a"] + (rows - 1) * nq * hd * 4, p["q"] + (rows - 1) * nq * hd * 4, kv[0].data_ptr(), kv[1].data_ptr(), pos + rows, nq, nkv, hd)
+            call(lib.forge_matmul_mat_packed, p["p"], rows, p["a"], packed["o"])
+            call(lib.forge_residual_add, x.data_ptr(), p["p"], rows * h)
+            call(lib.forge_rms_norm, p["y"], x.data_ptr(), norm.data_ptr(), rows, h, 1e-5)
+            call(lib.forge_matmul_mat_packed, p["g"], rows, p["y"], packed["gate"])
+            call(lib.forge_matmul_mat_packed, p["u"], rows, p["y"], packed["up"])
+            call(lib.forge_silu_mul, p["g"], p["g"], p["u"], rows * ff)
+            call(lib.forge_matmul_mat_packed, p["p"], rows, p["g"], packed["down"])
+            call(lib.forge_residual_add, x.data_ptr(), p["p"], rows * h)
+            pos += rows
+        return x.cpu().numpy(), kv.cpu().numpy()
+
+    want = layers(True)
+    assert np.isfinite(want[0]).all()
+    for _ in range(5):
+        got = layers(False)
+        assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+    for q in packed.values():
+        lib.forge_packed_destroy(q)
