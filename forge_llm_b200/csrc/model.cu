@@ -1293,7 +1293,11 @@ int32_t forge_step(ForgeModel* m, ForgeKV* kv, const ForgeStepEntry* entries, in
 }
 
 static int32_t ensure_hist(ForgeModel* m, int n) {
-    if (n > m->hist_cap) { FORGE_TRY(dev_alloc(m, &m->d_hist, size_t(n))); m->hist_cap = n; }
+    if (n > m->hist_cap) {
+        FORGE_TRY(dev_alloc(m, &m->d_hist, size_t(n)));
+        m->hist_cap = n;
+        ++m->scratch_gen;   // a captured step holds the address
+    }
     return FORGE_OK;
 }
 

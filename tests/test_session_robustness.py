@@ -46,6 +46,26 @@ def test_scratch_growth_between_caches(oracle):
     kv1.close(); kv4.close(); gm.close()
 
 
+@pytest.mark.parametrize("batch", [1, 3])
+def test_longer_request_after_a_captured_step(batch):
+    """A step is captured with the place of the tokens it records; a request for more tokens than any before has a new one, and its tokens are those of a first request."""
+    from forge_llm_b200 import runtime
+    c, blob, toks = _tiny()
+    out = []
+    for first in (None, 4):
+        gm = runtime.Model(c, blob)
+        kv = gm.new_cache(max_seq=128, batch=batch)
+        for n in ([first] if first else []) + [60]:
+            kv.reset()
+            for b in range(batch):
+                gm.forward_prefill(toks[: 20 + b], kv, seq=b)
+            got = gm.decode_greedy_batch([int(toks[b]) for b in range(batch)], n, kv)
+        out.append(np.array(got))
+        kv.close()
+        gm.close()
+    assert np.array_equal(out[0], out[1])
+
+
 def test_peer_sum_that_never_arrives_reports_timeout():
     """Tensor-parallel decode over peer memory on ONE GPU: rank 0 of a two-rank cut is attached to an exchange in which
     the slot of rank 1 is its own buffer, so nobody ever pushes rank 1's partial sums.  The consumer's bounded wait runs
