@@ -474,6 +474,20 @@ int32_t decode_launches_gemm(ForgeModel* m, ForgeKV* kv, int batch, bool greedy,
     return step_advance(kv->d_seq_len, n, m->d_step, st, nullptr);
 }
 
+// Whether a step of 2 .. 8 sequences takes the tcgen05 products (their weight-streaming form, operands and sums by the prompt's passes) instead of the mma.sync streaming
+// product, which the ranks of a tensor-parallel step need and which goes row by row of packed activations.  us per step of four layers at 2 / 4 / 5 / 8 sequences, mma.sync
+// against tcgen05: 135M shapes in Q8_0 160 / 162 / 191 / 192 against 140 / 145 / 146 / 149, 1B in Q4_0 311 / 317 / 373 / 386 against 295 / 297 / 301 / 304, 0.5B in Q8_0
+// 351 / 352 / 434 / 434 against 210 - 214, 7B in Q8_0 487 / 488 / 566 / 589 against 470 - 483.  Only with Q4_0 weights of which one product is more than one round of row tiles
+// over the SMs is the former ahead, up to four sequences, for which it packs half a tile (7B: 435 / 444 / 508 / 528 against 487 / 492 / 494 / 502).
+bool rows_by_gemm(const ForgeModel* m, int batch) {
+    if (m->cfg.tp_world > 1 || m->gemm_passes != 3 || !m->lm_head.qs || !gemm_tc5_supported(m->lm_head)) return false;
+    for (const ForgeLayer& L : m->layers)
+        if (!gemm_tc5_supported(L.qkv) || !gemm_tc5_supported(L.o) || !gemm_tc5_supported(L.gateup) || !gemm_tc5_supported(L.down)) return false;
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device);
+    return batch > 4 || m->cfg.quant == FORGE_Q8_0 || (2 * m->ff + 127) / 128 <= sms;
+}
+
 int32_t decode_launches(ForgeModel* m, ForgeKV* kv, int batch, bool greedy, bool record, const PrefillToken* pt = nullptr) {
     if (m->stack) return stack_decode_launches(m, kv, batch, greedy, record);
     const ForgeModelConfig& c = m->cfg;
@@ -508,9 +522,7 @@ int32_t decode_launches(ForgeModel* m, ForgeKV* kv, int batch, bool greedy, bool
         return gemv_tc(w, EPI_TP_PUSH, a, m->split, m->d_err, st);
     };
     if (batch >= 2 && !pt && m->uniform_basic && !m->trace_on) {
-        // up to 8 sequences: the mma.sync streaming product; beyond: the tcgen05 products (their weight-streaming form up to
-        // 32 rows, measured faster from about 16 rows on; the tile form for more)
-        if (batch > kBatchGroup / 2 && m->lm_head.qs) return decode_launches_gemm(m, kv, batch, greedy, record);
+        if (batch > kBatchGroup / 2 ? m->lm_head.qs != nullptr : rows_by_gemm(m, batch)) return decode_launches_gemm(m, kv, batch, greedy, record);
         return decode_launches_batched(m, kv, batch, greedy, record);
     }
     FORGE_TRY(embedding_rows(m->d_hidden, m->embed, pt ? pt->tok : m->d_tok, batch, m->h, record ? m->d_hist : nullptr, m->d_step, st));
