@@ -48,10 +48,10 @@ __global__ void rms_norm_kernel(OutT* out, __half* lo, const float* in, const fl
     }
 }
 
-// fp16 hi/lo output for rows of at most 256 * 4 * NV floats: the row is read once with 128-bit loads and stays in
+// f32, or fp16 hi/lo output for rows of at most 256 * 4 * NV floats: the row is read once with 128-bit loads and stays in
 // registers between the sum of squares and the scaling
-template <int NV>
-__global__ void __launch_bounds__(256) rms_norm_f16_vec_kernel(__half* out, __half* lo, const float* in, const float* w, int n, float eps) {
+template <int NV, typename OutT>
+__global__ void __launch_bounds__(256) rms_norm_vec_kernel(OutT* out, __half* lo, const float* in, const float* w, int n, float eps) {
     __shared__ float red[32];
     pdl_wait();
     pdl_trigger();
@@ -72,8 +72,12 @@ __global__ void __launch_bounds__(256) rms_norm_f16_vec_kernel(__half* out, __ha
         if (e >= n) continue;
         const float4 ww = *reinterpret_cast<const float4*>(w + e);
         const float r[4] = {v[i].x * inv * ww.x, v[i].y * inv * ww.y, v[i].z * inv * ww.z, v[i].w * inv * ww.w};
-        const __half2 h0 = __floats2half2_rn(r[0], r[1]), h1 = __floats2half2_rn(r[2], r[3]);
         const size_t o = size_t(blockIdx.x) * n + e;
+        if constexpr (sizeof(OutT) == 4) {
+            *reinterpret_cast<float4*>(out + o) = make_float4(r[0], r[1], r[2], r[3]);
+            continue;
+        }
+        const __half2 h0 = __floats2half2_rn(r[0], r[1]), h1 = __floats2half2_rn(r[2], r[3]);
         *reinterpret_cast<uint2*>(out + o) = make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
         if (lo) {
             const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
@@ -131,13 +135,25 @@ __global__ void __launch_bounds__(256) add_parts_norm_kernel(float* hidden, cons
     }
 }
 
-// thread per (row, head, pair): adjacent-pair rotation, table = {cos, sin}[pos][hd/2]
+// thread per (row, head, pair): adjacent-pair rotation, table = {cos, sin}[pos][hd/2]; two pairs of a head per thread where a head has an even number of them
 __global__ void rope_kernel(float* data, int rows, int base_pos, int hd, int heads, const float2* table) {
     pdl_wait();
     pdl_trigger();
-    int half = hd / 2;
-    long total = long(rows) * heads * half;
-    for (long i = blockIdx.x * long(blockDim.x) + threadIdx.x; i < total; i += long(gridDim.x) * blockDim.x) {
+    const int half = hd / 2;
+    const long i0 = blockIdx.x * long(blockDim.x) + threadIdx.x, step = long(gridDim.x) * blockDim.x;
+    if (half % 2 == 0 && !((reinterpret_cast<uintptr_t>(data) | reinterpret_cast<uintptr_t>(table)) & 15) && long(rows) * heads * (half / 2) < (1l << 31)) {
+        const unsigned quarter = unsigned(half / 2), total = unsigned(rows) * heads * quarter;
+        for (unsigned i = unsigned(i0); i < total; i += unsigned(step)) {
+            const unsigned rh = i / quarter, pr = i - rh * quarter;
+            const float4 cs = *reinterpret_cast<const float4*>(table + size_t(base_pos + rh / unsigned(heads)) * half + 2 * pr);
+            float4* p = reinterpret_cast<float4*>(data) + i;
+            const float4 v = *p;
+            *p = make_float4(v.x * cs.x - v.y * cs.y, v.x * cs.y + v.y * cs.x, v.z * cs.z - v.w * cs.w, v.z * cs.w + v.w * cs.z);
+        }
+        return;
+    }
+    const long total = long(rows) * heads * half;
+    for (long i = i0; i < total; i += step) {
         int pr = int(i % half);
         long rh = i / half;
         int r = int(rh / heads);
@@ -148,10 +164,23 @@ __global__ void rope_kernel(float* data, int rows, int base_pos, int hd, int hea
     }
 }
 
+// (the operators below take four values per thread where addresses and counts allow: memory-bound passes, whose loads were four bytes a thread)
+__device__ __forceinline__ bool four_wide(const void* a, const void* b, const void* c, size_t n) {
+    return !((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15) && n % 4 == 0;
+}
 __global__ void silu_mul_kernel(float* out, const float* g, const float* u, size_t n) {
     pdl_wait();
     pdl_trigger();
-    for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
+    const size_t i0 = blockIdx.x * size_t(blockDim.x) + threadIdx.x, step = size_t(gridDim.x) * blockDim.x;
+    if (four_wide(out, g, u, n)) {
+        for (size_t i = i0; i < n / 4; i += step) {
+            const float4 x = reinterpret_cast<const float4*>(g)[i], y = reinterpret_cast<const float4*>(u)[i];
+            reinterpret_cast<float4*>(out)[i] = make_float4((x.x / (1.0f + expf(-x.x))) * y.x, (x.y / (1.0f + expf(-x.y))) * y.y, (x.z / (1.0f + expf(-x.z))) * y.z,
+                                                            (x.w / (1.0f + expf(-x.w))) * y.w);
+        }
+        return;
+    }
+    for (size_t i = i0; i < n; i += step) {
         float x = g[i];
         out[i] = (x / (1.0f + expf(-x))) * u[i];
     }
@@ -168,7 +197,15 @@ __global__ void silu_mul_f16_kernel(__half* out, __half* lo, const float2* gu, s
 __global__ void residual_add_kernel(float* a, const float* b, size_t n) {
     pdl_wait();
     pdl_trigger();
-    for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) a[i] += b[i];
+    const size_t i0 = blockIdx.x * size_t(blockDim.x) + threadIdx.x, step = size_t(gridDim.x) * blockDim.x;
+    if (four_wide(a, b, a, n)) {
+        for (size_t i = i0; i < n / 4; i += step) {
+            const float4 x = reinterpret_cast<const float4*>(a)[i], y = reinterpret_cast<const float4*>(b)[i];
+            reinterpret_cast<float4*>(a)[i] = make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w);
+        }
+        return;
+    }
+    for (size_t i = i0; i < n; i += step) a[i] += b[i];
 }
 
 __global__ void embedding_kernel(float* out, const float* table, const uint32_t* tokens, int h, uint32_t* hist, const int32_t* step) {
@@ -435,7 +472,19 @@ __global__ void argmax_slices_kernel(uint32_t* result, const float* logits, int 
 __global__ void f32_to_f16_kernel(__half* out, __half* lo, const float* in, size_t n) {
     pdl_wait();
     pdl_trigger();
-    for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) store_split(out, lo, i, in[i]);
+    const size_t i0 = blockIdx.x * size_t(blockDim.x) + threadIdx.x, step = size_t(gridDim.x) * blockDim.x;
+    if (lo && four_wide(out, lo, in, n)) {
+        for (size_t i = i0; i < n / 4; i += step) {
+            const float4 v = reinterpret_cast<const float4*>(in)[i];
+            const __half2 h0 = __floats2half2_rn(v.x, v.y), h1 = __floats2half2_rn(v.z, v.w);
+            const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
+            const __half2 l0 = __floats2half2_rn(v.x - f0.x, v.y - f0.y), l1 = __floats2half2_rn(v.z - f1.x, v.w - f1.y);
+            reinterpret_cast<uint2*>(out)[i] = make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
+            reinterpret_cast<uint2*>(lo)[i] = make_uint2(*reinterpret_cast<const uint32_t*>(&l0), *reinterpret_cast<const uint32_t*>(&l1));
+        }
+        return;
+    }
+    for (size_t i = i0; i < n; i += step) store_split(out, lo, i, in[i]);
 }
 
 // -log p(target) of one logits row: log_z = max + ln(sum exp((l - max) as f64)) as the reference's corpus scorer forms it
@@ -489,15 +538,19 @@ inline int grid_for(size_t n, int threads = 256) {
 
 int32_t rms_norm_f32(float* out, const float* in, const float* w, int rows, int n, float eps, cudaStream_t st) {
     if (rows <= 0) return FORGE_OK;
-    FORGE_CUDA(launch_pdl(rms_norm_kernel<float>, dim3(rows), dim3(256), 0, st, out, nullptr, in, w, n, eps));
+    const bool aligned = !((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(w)) & 15) && n % 4 == 0;
+    if (aligned && n <= 2048) FORGE_CUDA(launch_pdl(rms_norm_vec_kernel<2, float>, dim3(rows), dim3(256), 0, st, out, nullptr, in, w, n, eps));
+    else if (aligned && n <= 4096) FORGE_CUDA(launch_pdl(rms_norm_vec_kernel<4, float>, dim3(rows), dim3(256), 0, st, out, nullptr, in, w, n, eps));
+    else if (aligned && n <= 8192) FORGE_CUDA(launch_pdl(rms_norm_vec_kernel<8, float>, dim3(rows), dim3(256), 0, st, out, nullptr, in, w, n, eps));
+    else FORGE_CUDA(launch_pdl(rms_norm_kernel<float>, dim3(rows), dim3(256), 0, st, out, nullptr, in, w, n, eps));
     FORGE_LAUNCH_CHECK();
     return FORGE_OK;
 }
 int32_t rms_norm_f16(__half* out, __half* lo, const float* in, const float* w, int rows, int n, float eps, cudaStream_t st) {
     if (rows <= 0) return FORGE_OK;
-    if (n % 4 == 0 && n <= 2048) FORGE_CUDA(launch_pdl(rms_norm_f16_vec_kernel<2>, dim3(rows), dim3(256), 0, st, out, lo, in, w, n, eps));
-    else if (n % 4 == 0 && n <= 4096) FORGE_CUDA(launch_pdl(rms_norm_f16_vec_kernel<4>, dim3(rows), dim3(256), 0, st, out, lo, in, w, n, eps));
-    else if (n % 4 == 0 && n <= 8192) FORGE_CUDA(launch_pdl(rms_norm_f16_vec_kernel<8>, dim3(rows), dim3(256), 0, st, out, lo, in, w, n, eps));
+    if (n % 4 == 0 && n <= 2048) FORGE_CUDA(launch_pdl(rms_norm_vec_kernel<2, __half>, dim3(rows), dim3(256), 0, st, out, lo, in, w, n, eps));
+    else if (n % 4 == 0 && n <= 4096) FORGE_CUDA(launch_pdl(rms_norm_vec_kernel<4, __half>, dim3(rows), dim3(256), 0, st, out, lo, in, w, n, eps));
+    else if (n % 4 == 0 && n <= 8192) FORGE_CUDA(launch_pdl(rms_norm_vec_kernel<8, __half>, dim3(rows), dim3(256), 0, st, out, lo, in, w, n, eps));
     else FORGE_CUDA(launch_pdl(rms_norm_kernel<__half>, dim3(rows), dim3(256), 0, st, out, lo, in, w, n, eps));
     FORGE_LAUNCH_CHECK();
     return FORGE_OK;
@@ -515,13 +568,13 @@ int32_t add_parts_rms_norm_f16(float* hidden, const float* parts, int nparts, si
 int32_t rope_rows(float* data, int rows, int base_pos, int head_dim, int heads, const float* table, cudaStream_t st) {
     size_t n = size_t(rows) * heads * (head_dim / 2);
     if (n == 0) return FORGE_OK;
-    FORGE_CUDA(launch_pdl(rope_kernel, dim3(grid_for(n)), dim3(256), 0, st, data, rows, base_pos, head_dim, heads, reinterpret_cast<const float2*>(table)));
+    FORGE_CUDA(launch_pdl(rope_kernel, dim3(grid_for((n + 1) / 2)), dim3(256), 0, st, data, rows, base_pos, head_dim, heads, reinterpret_cast<const float2*>(table)));
     FORGE_LAUNCH_CHECK();
     return FORGE_OK;
 }
 int32_t silu_mul_f32(float* out, const float* g, const float* u, size_t n, cudaStream_t st) {
     if (n == 0) return FORGE_OK;
-    FORGE_CUDA(launch_pdl(silu_mul_kernel, dim3(grid_for(n)), dim3(256), 0, st, out, g, u, n));
+    FORGE_CUDA(launch_pdl(silu_mul_kernel, dim3(grid_for((n + 3) / 4)), dim3(256), 0, st, out, g, u, n));
     FORGE_LAUNCH_CHECK();
     return FORGE_OK;
 }
@@ -534,7 +587,7 @@ int32_t silu_mul_f16(__half* out, __half* lo, const float* gu, int rows, int ffn
 }
 int32_t residual_add_f32(float* a, const float* b, size_t n, cudaStream_t st) {
     if (n == 0) return FORGE_OK;
-    FORGE_CUDA(launch_pdl(residual_add_kernel, dim3(grid_for(n)), dim3(256), 0, st, a, b, n));
+    FORGE_CUDA(launch_pdl(residual_add_kernel, dim3(grid_for((n + 3) / 4)), dim3(256), 0, st, a, b, n));
     FORGE_LAUNCH_CHECK();
     return FORGE_OK;
 }
@@ -629,7 +682,7 @@ int32_t q8_round_f16(__half* hi, __half* lo, size_t n, cudaStream_t st) {
 
 int32_t f32_to_f16(__half* out, __half* lo, const float* in, size_t n, cudaStream_t st) {
     if (n == 0) return FORGE_OK;
-    FORGE_CUDA(launch_pdl(f32_to_f16_kernel, dim3(grid_for(n)), dim3(256), 0, st, out, lo, in, n));
+    FORGE_CUDA(launch_pdl(f32_to_f16_kernel, dim3(grid_for((n + 3) / 4)), dim3(256), 0, st, out, lo, in, n));
     FORGE_LAUNCH_CHECK();
     return FORGE_OK;
 }

@@ -418,3 +418,68 @@ def test_operators_in_a_row_see_each_other(L, rows):
         assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
     for q in packed.values():
         lib.forge_packed_destroy(q)
+
+
+@pytest.mark.parametrize("n", [4, 1000, 4097, 8192, 1300000])
+def test_wide_and_narrow_operators_agree(L, n):
+    """Buffers that begin on sixteen bytes and counts of whole fours take wider loads: the same bits as one float further on, and nothing outside is written."""
+    import torch
+    lib, check = L
+    rng = np.random.default_rng(n)
+    g, u = rng.standard_normal(n, dtype=np.float32) * 4, rng.standard_normal(n, dtype=np.float32)
+    res = []
+    for skew in (0, 1):
+        b = [torch.full((n + 8,), 7.0, device="cuda") for _ in range(3)]
+        v = [x[skew:skew + n] for x in b]
+        v[0].copy_(torch.from_numpy(g))
+        v[1].copy_(torch.from_numpy(u))
+        check(lib.forge_silu_mul(v[2].data_ptr(), v[0].data_ptr(), v[1].data_ptr(), n, None))
+        check(lib.forge_residual_add(v[0].data_ptr(), v[1].data_ptr(), n, None))
+        _sync()
+        assert all(x[skew + n:].eq(7.0).all() and x[:skew].eq(7.0).all() for x in b)
+        res.append((v[0].cpu().numpy(), v[2].cpu().numpy()))
+    assert np.array_equal(res[0][0], g + u) and np.array_equal(res[0][1], res[1][1]) and np.array_equal(res[1][0], g + u)
+    ref = g.astype(np.float64) / (1 + np.exp(-g.astype(np.float64))) * u
+    assert rel_l2(res[0][1], ref) < 3e-7
+
+
+@pytest.mark.parametrize("rows,n", [(1, 4), (3, 1023), (2, 1024), (2, 2052), (2, 4100), (1, 8192), (2, 8196)])
+def test_rms_norm_forms(L, rows, n):
+    """Row lengths around the register forms' limits, buffers on and off sixteen bytes, against 64 bits; f32 sums of n terms in some order owe a few ulp."""
+    import torch
+    lib, check = L
+    rng = np.random.default_rng(n)
+    x, w = rng.standard_normal((rows, n), dtype=np.float32) * 3, rng.standard_normal(n, dtype=np.float32)
+    ref = x / np.sqrt((x.astype(np.float64) ** 2).mean(1, keepdims=True) + 1e-5) * w
+    for skew in (0, 1):
+        b = [torch.full((rows * n + 8,), 7.0, device="cuda") for _ in range(2)]
+        v = [t[skew:skew + rows * n] for t in b]
+        v[0].copy_(torch.from_numpy(x.ravel()))
+        check(lib.forge_rms_norm(v[1].data_ptr(), v[0].data_ptr(), dev(w).data_ptr(), rows, n, C.c_float(1e-5), None))
+        _sync()
+        assert rel_l2(v[1].cpu().numpy().reshape(rows, n), ref) < 1e-6
+        assert b[1][skew + rows * n:].eq(7.0).all() and b[1][:skew].eq(7.0).all()
+
+
+@pytest.mark.parametrize("hd,heads,rows", [(64, 9, 1), (34, 3, 5), (2, 4, 3), (96, 4, 700)])
+def test_rope_forms(L, oracle, hd, heads, rows):
+    import torch
+    lib, check = L
+    rng = np.random.default_rng(hd)
+    x = rng.standard_normal((rows, heads * hd), dtype=np.float32)
+    tab = np.empty((17 + rows, hd // 2, 2), np.float32)
+    check(lib.forge_rope_table(tab.ctypes.data_as(C.c_void_p), 17 + rows, hd, C.c_float(1e4)))
+    dt = dev(tab)
+    p = x.reshape(rows, heads, hd // 2, 2).astype(np.float64)
+    cs = tab[17:, None].astype(np.float64)
+    ref = np.stack([p[..., 0] * cs[..., 0] - p[..., 1] * cs[..., 1], p[..., 0] * cs[..., 1] + p[..., 1] * cs[..., 0]], -1).reshape(rows, -1)
+    got = []
+    for skew in (0, 2):
+        b = torch.full((x.size + 8,), 7.0, device="cuda")
+        v = b[skew:skew + x.size]
+        v.copy_(torch.from_numpy(x.ravel()))
+        check(lib.forge_rope(v.data_ptr(), rows, 17, hd, heads, dt.data_ptr(), None))
+        _sync()
+        assert b[skew + x.size:].eq(7.0).all() and b[:skew].eq(7.0).all()
+        got.append(v.cpu().numpy().reshape(rows, -1))
+    assert np.array_equal(got[0], got[1]) and np.abs(got[0] - ref).max() < 2e-6
