@@ -314,7 +314,7 @@ bool gemm_tc5_supported(const QWeight& w);
 // fp16 hi (+ lo) rows [m][N / 2] and `out` is not written
 int32_t gemm_tc5(float* out, const __half* A, const __half* Alo, const QWeight& w, int m, const float* resid, int* err, cudaStream_t st,
                  int ksplit = 1, size_t part_stride = 0, __half* act_hi = nullptr, __half* act_lo = nullptr, int* parts = nullptr);
-int gemm_tc5_ksplit(const QWeight& w);
+int gemm_tc5_ksplit(const QWeight& w, int m);
 // The same product on CTA pairs (gemm_pair.cu; Q8_0 / Q4_0, split precision): tokens per tile, partial outputs part_stride apart that remain to be added, pairs
 // launched, and the microseconds that this should take.  K runs as ksplit slices; parts_only != 0 asks for that many partial outputs
 struct PairPlan { int nt = 0, parts = 1, pairs = 0; double cost = 0; };

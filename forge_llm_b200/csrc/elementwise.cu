@@ -99,11 +99,10 @@ __global__ void __launch_bounds__(256) add_parts_norm_kernel(float* hidden, cons
     float4 v[NV];
     float ss = 0.f;
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
+    for (int i = 0; i < NV; ++i) {   // no store between the loads: one memory round trip for the row
         const int e = (threadIdx.x + i * 256) * 4;
         v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (e < n) {
-            // all loads first (one memory round trip), then the sum in slice order
             v[i] = *reinterpret_cast<const float4*>(x + e);
             float4 a[4];
 #pragma unroll
@@ -111,9 +110,13 @@ __global__ void __launch_bounds__(256) add_parts_norm_kernel(float* hidden, cons
                 a[s] = s < nparts ? *reinterpret_cast<const float4*>(pr + size_t(s) * pstride + e) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
             for (int s = 0; s < 4; ++s) { v[i].x += a[s].x; v[i].y += a[s].y; v[i].z += a[s].z; v[i].w += a[s].w; }
-            *reinterpret_cast<float4*>(x + e) = v[i];
         }
         ss += v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
+    }
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int e = (threadIdx.x + i * 256) * 4;
+        if (e < n) *reinterpret_cast<float4*>(x + e) = v[i];
     }
     if (!w) return;
     ss = block_sum(ss, red);
@@ -313,29 +316,42 @@ __global__ void qkv_post_kernel(const float* qkv, int nparts, size_t pstride, in
     const float2* src = reinterpret_cast<const float2*>(qkv + size_t(r) * (qk + 2 * kv));
     const int lp = pos / FORGE_KV_PAGE;
     const size_t prow = (size_t(page_row ? page_row[lp] : lp) * FORGE_KV_PAGE + pos % FORGE_KV_PAGE) * kv;
-    for (int i = threadIdx.x; i < npairs; i += blockDim.x) {
-        float2 v = src[i];
-        for (int s = 1; s < nparts; ++s) {
-            const float2 a = reinterpret_cast<const float2*>(qkv + size_t(s) * pstride + size_t(r) * (qk + 2 * kv))[i];
-            v.x += a.x; v.y += a.y;
-        }
-        int col = 2 * i;
-        if (bias) { v.x += bias[col]; v.y += bias[col + 1]; }
-        int region = 0;
-        if (col >= qk) { col -= qk; region = 1; }
-        if (region == 1 && col >= kv) { col -= kv; region = 2; }
-        if (region < 2) {
-            float2 cs = rope[size_t(pos) * (hd / 2) + (col % hd) / 2];
-            v = make_float2(v.x * cs.x - v.y * cs.y, v.x * cs.y + v.y * cs.x);
-        }
-        __half2 hv = __floats2half2_rn(v.x, v.y);
-        if (region == 0) {
-            *reinterpret_cast<__half2*>(q16 + size_t(r) * qk + col) = hv;
-            if (q16_lo) {  // the part of the query fp16 drops, for the precise attention
-                const float2 hf = __half22float2(hv);
-                *reinterpret_cast<__half2*>(q16_lo + size_t(r) * qk + col) = __floats2half2_rn(v.x - hf.x, v.y - hf.y);
+    constexpr int kAhead = 4;   // pairs of a thread that are loaded in front of the first store
+    for (int i0 = threadIdx.x; i0 < npairs; i0 += kAhead * blockDim.x) {
+        float2 v[kAhead], cs[kAhead], bs[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const int i = i0 + u * int(blockDim.x), col = 2 * i;
+            if (i >= npairs) break;
+            v[u] = src[i];
+            bs[u] = bias ? make_float2(bias[col], bias[col + 1]) : make_float2(0.f, 0.f);
+            cs[u] = col < qk + kv ? rope[size_t(pos) * (hd / 2) + ((col < qk ? col : col - qk) % hd) / 2] : make_float2(1.f, 0.f);
+            for (int s = 1; s < nparts; ++s) {
+                const float2 a = reinterpret_cast<const float2*>(qkv + size_t(s) * pstride + size_t(r) * (qk + 2 * kv))[i];
+                v[u].x += a.x; v[u].y += a.y;
             }
-        } else *reinterpret_cast<__half2*>((region == 1 ? k_pool : v_pool) + prow + col) = hv;
+        }
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const int i = i0 + u * int(blockDim.x);
+            if (i >= npairs) break;
+            int col = 2 * i;
+            float2 x = v[u];
+            if (bias) { x.x += bs[u].x; x.y += bs[u].y; }
+            if (col < qk + kv) x = make_float2(x.x * cs[u].x - x.y * cs[u].y, x.x * cs[u].y + x.y * cs[u].x);
+            const __half2 hv = __floats2half2_rn(x.x, x.y);
+            if (col < qk) {
+                *reinterpret_cast<__half2*>(q16 + size_t(r) * qk + col) = hv;
+                if (q16_lo) {  // the part of the query fp16 drops, for the precise attention
+                    const float2 hf = __half22float2(hv);
+                    *reinterpret_cast<__half2*>(q16_lo + size_t(r) * qk + col) = __floats2half2_rn(x.x - hf.x, x.y - hf.y);
+                }
+            } else {
+                col -= qk;
+                const bool is_v = col >= kv;
+                *reinterpret_cast<__half2*>((is_v ? v_pool : k_pool) + prow + (is_v ? col - kv : col)) = hv;
+            }
+        }
     }
 }
 

@@ -718,7 +718,16 @@ bool gemm_tc5_supported(const QWeight& w) { return w.K % BK == 0 && w.K >= BK; }
 // keep at least 16 K steps (1024 columns) per slice, at most 4.  A tensor-memory accumulator rounds toward zero at every
 // accumulation, a bias that grows with the chain (measured: 7e-6 of the result at K = 2048, 2.7e-5 at K = 8192) and,
 // being one-sided, adds up over the layers; shorter chains keep it at the K = 2048 level.
-int gemm_tc5_ksplit(const QWeight& w) { return std::max(1, std::min(4, w.K / 1024)); }
+// A few rows leave most of the chip without a tile: there slices are halved while their tiles still fit one round and keep three K steps, to four at most (a step of
+// eight sequences through four layers: 135M shapes 149 -> 127 us, 0.5B 214 -> 194, 1B 304 -> 286).
+int gemm_tc5_ksplit(const QWeight& w, int m) {
+    int ks = std::max(1, std::min(4, w.K / 1024)), dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const long tiles = m <= 32 ? (w.N + 127) / 128 : 2l * ((w.N + 255) / 256) * ((m + 95) / 96);   // (a pair's tile takes two SMs)
+    while (ks <= 2 && 2 * ks * tiles <= sms && w.K / BK >= 6 * ks) ks *= 2;
+    return ks;
+}
 
 int32_t gemm_tc5(float* out, const __half* A, const __half* Alo, const QWeight& w, int m, const float* resid, int* err, cudaStream_t st,
                  int ksplit, size_t part_stride, __half* act_hi, __half* act_lo, int* parts) {

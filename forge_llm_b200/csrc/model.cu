@@ -220,7 +220,7 @@ int32_t row_sliced_gemm(ForgeModel* m, const QWeight& w, const __half* a, const 
 // itself (residual add + RMSNorm fused, emit.rs:455-459 and :327-334): shorter accumulation chains in tensor memory
 // and more CTAs for these few-row-tile matrices.
 int32_t row_sliced_gemm_norm(ForgeModel* m, const QWeight& w, const __half* a, const __half* alo, int n, const float* next_norm, __half* nlo, cudaStream_t st) {
-    const int ks = gemm_tc5_ksplit(w);
+    const int ks = gemm_tc5_ksplit(w, n);
     if (m->cfg.tp_world == 1 && gemm_tc5_supported(w) && m->p_parts) {
         const size_t stride = size_t(n) * m->h;
         int parts;
@@ -284,7 +284,7 @@ int32_t prefill_seq(ForgeModel* m, ForgeKV* kv, int seq, const uint32_t* tokens_
         // K and V are rounded to fp16 on their way into the cache, which turns a difference of e before the rounding into
         // ~sqrt(e * 2^-11) after it: the QKV product therefore runs as K slices (shorter accumulation chains in tensor
         // memory, see gemm_tc5_ksplit) whose partials the epilogue kernel adds
-        const int qks = (m->cfg.tp_world == 1 && gemm_tc5_supported(L.qkv) && m->p_qkv_parts) ? std::max(1, std::min(4, L.qkv.K / 1024)) : 1;
+        const int qks = (m->cfg.tp_world == 1 && gemm_tc5_supported(L.qkv) && m->p_qkv_parts) ? gemm_tc5_ksplit(L.qkv, n) : 1;
         const size_t qstride = size_t(n) * (m->qk + 2 * m->kv);
         int qparts = 1;
         if (qks > 1) FORGE_TRY(gemm_tc5(m->p_qkv_parts, m->p_normed, nlo, L.qkv, n, nullptr, m->d_err, st, qks, qstride, nullptr, nullptr, &qparts));
@@ -453,7 +453,7 @@ int32_t decode_launches_gemm(ForgeModel* m, ForgeKV* kv, int batch, bool greedy,
         __half* kp = kv->k_pool + size_t(l) * kv->layer_stride;
         __half* vp = kv->v_pool + size_t(l) * kv->layer_stride;
         // q/k/v as K slices like the prompt's (more CTAs for a product of few row tiles; the epilogue adds the slices)
-        const int qks = (c.tp_world == 1 && split && gemm_tc5_supported(L.qkv) && m->p_qkv_parts) ? std::max(1, std::min(4, L.qkv.K / 1024)) : 1;
+        const int qks = (c.tp_world == 1 && split && gemm_tc5_supported(L.qkv) && m->p_qkv_parts) ? gemm_tc5_ksplit(L.qkv, n) : 1;
         const size_t qstride = size_t(n) * (m->qk + 2 * m->kv);
         int qparts = 1;
         if (qks > 1) FORGE_TRY(gemm_tc5(m->p_qkv_parts, m->p_normed, nlo, L.qkv, n, nullptr, m->d_err, st, qks, qstride, nullptr, nullptr, &qparts));
