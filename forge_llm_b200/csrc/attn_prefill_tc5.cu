@@ -21,6 +21,9 @@
 // only a few times per row.  Tensor memory: S [0,64), P0 [64,128), P1 [128,192) (hi | lo halves), O from 192: 256 columns
 // for 64-wide heads (two CTAs per SM), 512 for wider ones (one CTA per SM, which is also what their shared memory
 // allows).  Every wait is bounded; one that gives up sets the error word and the CTA still frees its tensor memory.
+//
+// A query tile's keys are one chain of about 1.1 us a tile, and the last query tile's chain is the whole launch where heads are few: there `split` CTAs, a cluster, take
+// the key tiles in turn, and each finishes a share of the dimensions from the others' sums, which they store into its shared memory (the ring, which is no longer needed).
 #include <cuda.h>
 
 #include <algorithm>
@@ -46,6 +49,7 @@ struct Tc5AttnParams {
     AttnPrefillArgs a;
     float scale_log2;     // 1/sqrt(head_dim) * log2(e)
     int* err;
+    int split;            // CTAs per query tile (1, 2, 4)
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
@@ -133,8 +137,74 @@ __device__ __forceinline__ uint32_t pack_h2_lo(float a, float b, uint32_t hi) { 
     return pack_h2(a - hf.x, b - hf.y);
 }
 
-// HD: head_dim (64, 96, 128); SW: sliding window; PRECISE: hi + lo operands
-template <int HD, bool SW, bool PRECISE>
+// eight finished values of an output row
+__device__ __forceinline__ void put8(const AttnPrefillArgs& a, size_t at, const float (&x)[8]) {
+    if (a.out32) {
+        *reinterpret_cast<float4*>(a.out32 + at) = make_float4(x[0], x[1], x[2], x[3]);
+        *reinterpret_cast<float4*>(a.out32 + at + 4) = make_float4(x[4], x[5], x[6], x[7]);
+    } else {
+        uint32_t hi[4], lo[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            hi[e] = pack_h2(x[2 * e], x[2 * e + 1]);
+            lo[e] = pack_h2_lo(x[2 * e], x[2 * e + 1], hi[e]);
+        }
+        *reinterpret_cast<uint4*>(a.out16 + at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        if (a.out16_lo) *reinterpret_cast<uint4*>(a.out16_lo + at) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    }
+}
+// The sums of a query tile's CTAs (row r of each in the thread of the same number) become its output: every CTA hands each other one the dimensions that one finishes,
+// [CTA][four dimensions][row] behind [CTA][row]{reference maximum, sum}.
+template <int HD>
+__device__ __forceinline__ void merge_parts(const AttnPrefillArgs& a, unsigned char* buf, int rank, int split, uint32_t o_addr, bool any, int r, float m, float l, bool live, size_t row_off) {
+    const int share = HD / split;   // 16 .. 64, a multiple of eight
+    float2* const ml = reinterpret_cast<float2*>(buf);
+    float4* const part = reinterpret_cast<float4*>(buf + 4 * BM * 8);
+    tc5::cluster_sync();   // nobody's ring is in use any more
+#pragma unroll
+    for (int c0 = 0; c0 < HD; c0 += 16) {
+        uint32_t o[16];
+        tc5::tmem_ld16(o_addr + uint32_t(c0), o);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int i = 0; i < 16; i += 4) {
+            const int to = (c0 + i) / share, k = (c0 + i - to * share) / 4;
+            const float4 v = any ? make_float4(__uint_as_float(o[i]), __uint_as_float(o[i + 1]), __uint_as_float(o[i + 2]), __uint_as_float(o[i + 3])) : make_float4(0.f, 0.f, 0.f, 0.f);
+            tc5::cluster_store4(tc5::cluster_addr(part + (rank * (share / 4) + k) * BM + r, to), v);
+        }
+    }
+    for (int to = 0; to < split; ++to) {
+        const uint32_t at = tc5::cluster_addr(ml + rank * BM + r, to);
+        asm volatile("st.shared::cluster.v2.f32 [%0], {%1,%2};" ::"r"(at), "f"(m), "f"(l) : "memory");
+    }
+    tc5::cluster_sync();   // all parts are in place
+    float top = -INFINITY, f[4], sum = 0.f;
+    for (int s = 0; s < split; ++s) top = fmaxf(top, ml[s * BM + r].x);
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+        const float2 x = s < split ? ml[s * BM + r] : make_float2(-INFINITY, 0.f);
+        f[s] = x.x == -INFINITY ? 0.f : exp2f(x.x - top);
+        sum += x.y * f[s];
+    }
+    const float inv = sum > 0.f ? 1.0f / sum : 0.f;
+    if (!live) return;
+    for (int k = 0; k < share / 4; k += 2) {
+        float x[8] = {};
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            if (s >= split) break;
+            const float4 u = part[(s * (share / 4) + k) * BM + r], v = part[(s * (share / 4) + k + 1) * BM + r];
+            x[0] = fmaf(u.x, f[s], x[0]); x[1] = fmaf(u.y, f[s], x[1]); x[2] = fmaf(u.z, f[s], x[2]); x[3] = fmaf(u.w, f[s], x[3]);
+            x[4] = fmaf(v.x, f[s], x[4]); x[5] = fmaf(v.y, f[s], x[5]); x[6] = fmaf(v.z, f[s], x[6]); x[7] = fmaf(v.w, f[s], x[7]);
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] *= inv;
+        put8(a, row_off + rank * share + 4 * k, x);
+    }
+}
+
+// HD: head_dim (64, 96, 128); SW: sliding window; PRECISE: hi + lo operands; PARTS: several CTAs per query tile
+template <int HD, bool SW, bool PRECISE, bool PARTS>
 __global__ void __launch_bounds__(kThreads) attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_qlo,
                                                                      const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                                                                      Tc5AttnParams p) {
@@ -155,14 +225,15 @@ __global__ void __launch_bounds__(kThreads) attn_prefill_tc5_kernel(const __grid
     const AttnPrefillArgs& a = p.a;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // CTAs in the order of their work: all heads of the last query tile (the most key tiles) first, the first tile last
-    const int linear = int(blockIdx.x + gridDim.x * blockIdx.y);
-    const int h_ = linear % a.nq, tile = int(gridDim.x) - 1 - linear / a.nq;
+    const int split = PARTS ? p.split : 1, rank = PARTS ? int(blockIdx.x) % split : 0, tiles = int(gridDim.x) / split;
+    const int linear = int(blockIdx.x) / split + tiles * int(blockIdx.y);
+    const int h_ = linear % a.nq, tile = tiles - 1 - linear / a.nq;
     const int h = h_, kvh = h / (a.nq / a.nkv);
     const int q0 = tile * BM;
     const int q_last = min(q0 + BM, a.m) - 1;
     const int lp_last = (a.base_pos + q_last) / BN;
-    const int lp_first = (SW && a.base_pos + q0 - a.window + 1 > 0) ? (a.base_pos + q0 - a.window + 1) / BN : 0;
-    const int nblk = lp_last - lp_first + 1;
+    const int lp_begin = (SW && a.base_pos + q0 - a.window + 1 > 0) ? (a.base_pos + q0 - a.window + 1) / BN : 0;
+    const int lp_first = lp_begin + rank, nblk = lp_last < lp_first ? 0 : (lp_last - lp_first) / split + 1;   // this CTA's: every split-th
 
     if (tid == 0) {
         mbar_init(&q_full, 1);
@@ -195,7 +266,7 @@ __global__ void __launch_bounds__(kThreads) attn_prefill_tc5_kernel(const __grid
             for (int j = 0; j < nblk; ++j) {
                 const int s = j % KVS, use = j / KVS;
                 if (use > 0 && !mbar_wait(&kv_empty[s], (use - 1) & 1, &s_err)) { atomicExch(&s_err, 1); break; }
-                const int lp = lp_first + j;
+                const int lp = lp_first + j * split;
                 const int row = (a.page_row ? a.page_row[lp] : lp) * BN;
                 unsigned char* dst = sKV + size_t(s) * STAGE;
                 mbar_expect_tx(&kv_full[s], uint32_t(STAGE));
@@ -225,10 +296,10 @@ __global__ void __launch_bounds__(kThreads) attn_prefill_tc5_kernel(const __grid
                 }
                 __syncwarp();
             };
-            if (ok && tc5::all_lanes(mbar_wait(&kv_full[0], 0, &s_err))) {
+            if (nblk > 0 && ok && tc5::all_lanes(mbar_wait(&kv_full[0], 0, &s_err))) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 issue_s(0);
-            } else {
+            } else if (nblk > 0) {
                 ok = false;
             }
             for (int j = 0; j < nblk && ok; ++j) {
@@ -264,7 +335,7 @@ __global__ void __launch_bounds__(kThreads) attn_prefill_tc5_kernel(const __grid
         float m_ref = -INFINITY, l_run = 0.f;         // reference maximum (base-2 domain, scaled) and the sum relative to it
         bool ok = true;
         for (int j = 0; j < nblk; ++j) {
-            const int t0 = (lp_first + j) * BN;
+            const int t0 = (lp_first + j * split) * BN;
             if (ok && !mbar_wait(&s_full, j & 1, &s_err)) { atomicExch(&s_err, 1); ok = false; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             uint32_t sv[2][32];
@@ -332,39 +403,37 @@ __global__ void __launch_bounds__(kThreads) attn_prefill_tc5_kernel(const __grid
             if (lane == 0) mbar_arrive(&p_full[j & 1]);
         }
         // ---------------- the tile's output: O / l
-        if (ok && !mbar_wait(&pv_done[(nblk - 1) & 1], ((nblk - 1) >> 1) & 1, &s_err)) { atomicExch(&s_err, 1); ok = false; }
+        if (nblk > 0 && ok && !mbar_wait(&pv_done[(nblk - 1) & 1], ((nblk - 1) >> 1) & 1, &s_err)) { atomicExch(&s_err, 1); ok = false; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
         const int qr = q0 + r;
         const size_t row_off = (size_t(qr) * a.nq + h) * HD;
+        const bool live = qr < a.m && ok;
+        if constexpr (PARTS) {
+            merge_parts<HD>(a, sKV, rank, split, lane_addr + kColO, nblk > 0, r, m_ref, l_run, live, row_off);
+        } else {
+            const float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
 #pragma unroll
-        for (int c0 = 0; c0 < HD; c0 += 32) {
-            uint32_t o[32];
-            tmem_ld32(lane_addr + kColO + c0, o);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (qr < a.m && ok) {
-                if (a.out32) {
-#pragma unroll
-                    for (int i = 0; i < 32; i += 4)
-                        *reinterpret_cast<float4*>(a.out32 + row_off + c0 + i) =
-                            make_float4(__uint_as_float(o[i]) * inv, __uint_as_float(o[i + 1]) * inv, __uint_as_float(o[i + 2]) * inv, __uint_as_float(o[i + 3]) * inv);
-                } else {
+            for (int c0 = 0; c0 < HD; c0 += 32) {
+                uint32_t o[32];
+                tmem_ld32(lane_addr + kColO + c0, o);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (live) {
 #pragma unroll
                     for (int i = 0; i < 32; i += 8) {
-                        uint32_t hi[4], lo[4];
+                        float x[8];
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const float x0 = __uint_as_float(o[i + 2 * e]) * inv, x1 = __uint_as_float(o[i + 2 * e + 1]) * inv;
-                            hi[e] = pack_h2(x0, x1);
-                            lo[e] = pack_h2_lo(x0, x1, hi[e]);
-                        }
-                        *reinterpret_cast<uint4*>(a.out16 + row_off + c0 + i) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-                        if (a.out16_lo) *reinterpret_cast<uint4*>(a.out16_lo + row_off + c0 + i) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                        for (int e = 0; e < 8; ++e) x[e] = __uint_as_float(o[i + e]) * inv;
+                        put8(a, row_off + c0 + i, x);
                     }
                 }
             }
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    }
+    if (PARTS && warp < 2) {   // the softmax warps' meetings are the whole cluster's
+        __syncwarp();
+        tc5::cluster_sync();
+        tc5::cluster_sync();
     }
     __syncthreads();
     if (warp == 1) {
@@ -405,23 +474,38 @@ int32_t make_map3(CUtensorMap* map, const __half* base, int hd, int heads, size_
     return FORGE_OK;
 }
 
-template <int HD, bool SW, bool PRECISE>
+template <int HD, bool SW, bool PRECISE, bool PARTS>
 int32_t launch(const CUtensorMap& mq, const CUtensorMap& mql, const CUtensorMap& mk, const CUtensorMap& mv, const Tc5AttnParams& p, cudaStream_t st) {
     constexpr int NCH = (HD + 63) / 64;
     const size_t smem = size_t(PRECISE ? 2 : 1) * NCH * BM * 128 + size_t(KVS) * 2 * NCH * BN * 128 + 1024;
-    auto kern = attn_prefill_tc5_kernel<HD, SW, PRECISE>;
+    auto kern = attn_prefill_tc5_kernel<HD, SW, PRECISE, PARTS>;
     FORGE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    dim3 grid((p.a.m + BM - 1) / BM, p.a.nq);
-    FORGE_CUDA(launch_pdl(kern, grid, dim3(kThreads), smem, st, mq, mql, mk, mv, p));
+    dim3 grid((p.a.m + BM - 1) / BM * p.split, p.a.nq);
+    FORGE_CUDA(launch_pdl_cluster(kern, grid, dim3(kThreads), p.split, smem, st, mq, mql, mk, mv, p));
     FORGE_LAUNCH_CHECK();
     return FORGE_OK;
 }
 
-template <int HD>
+template <int HD, bool PARTS>
 int32_t launch_hd(const CUtensorMap& mq, const CUtensorMap& mql, const CUtensorMap& mk, const CUtensorMap& mv, const Tc5AttnParams& p, cudaStream_t st) {
     const bool sw = p.a.window > 0;
-    if (p.a.precise) return sw ? launch<HD, true, true>(mq, mql, mk, mv, p, st) : launch<HD, false, true>(mq, mql, mk, mv, p, st);
-    return sw ? launch<HD, true, false>(mq, mql, mk, mv, p, st) : launch<HD, false, false>(mq, mql, mk, mv, p, st);
+    if (p.a.precise) return sw ? launch<HD, true, true, PARTS>(mq, mql, mk, mv, p, st) : launch<HD, false, true, PARTS>(mq, mql, mk, mv, p, st);
+    return sw ? launch<HD, true, false, PARTS>(mq, mql, mk, mv, p, st) : launch<HD, false, false, PARTS>(mq, mql, mk, mv, p, st);
+}
+
+// CTAs per query tile: more while every CTA still has an SM of its own and four key tiles to do (us at 1 / 2 / 4: 33 rows behind 2000 positions with 32 heads of 64
+// 34.6 / 22.2 / 15.1, 1000 rows with 9 heads 21.0 / 15.2 / 18.0, 130 behind 1000 with 32 heads of 128 27.3 / 21.2 / 30.8, 100 rows with 9 heads 7.3 / 8.3 / 7.8;
+// beyond one per SM the softmax warps are what counts, and those of more CTAs only begin and end more often: 1000 rows with 32 heads 22.8 / 28.1)
+int prefill_split(const AttnPrefillArgs& a) {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const long ctas = long((a.m + BM - 1) / BM) * a.nq;
+    int longest = (a.base_pos + a.m + BN - 1) / BN;
+    if (a.window > 0) longest = std::min(longest, (a.window + BM - 2) / BN + 2);
+    int split = 1;
+    while (split < 4 && ctas * split * 2 <= sms && longest / (split * 2) >= 4) split *= 2;
+    return split;
 }
 
 }  // namespace
@@ -436,12 +520,12 @@ int32_t attn_prefill(const AttnPrefillArgs& a, cudaStream_t st) {
     FORGE_TRY(make_map3(&mql, a.precise ? a.q16_lo : a.q16, a.hd, a.nq, size_t(a.m), BM));
     FORGE_TRY(make_map3(&mk, a.k_pool, a.hd, a.nkv, a.pool_rows, BN));
     FORGE_TRY(make_map3(&mv, a.v_pool, a.hd, a.nkv, a.pool_rows, BN));
-    Tc5AttnParams p{a, 1.0f / sqrtf(float(a.hd)) * 1.4426950408889634f, a.err};
+    Tc5AttnParams p{a, 1.0f / sqrtf(float(a.hd)) * 1.4426950408889634f, a.err, prefill_split(a)};
     switch (a.hd) {
-        case 64: return launch_hd<64>(mq, mql, mk, mv, p, st);
-        case 96: return launch_hd<96>(mq, mql, mk, mv, p, st);
+        case 64: return p.split > 1 ? launch_hd<64, true>(mq, mql, mk, mv, p, st) : launch_hd<64, false>(mq, mql, mk, mv, p, st);
+        case 96: return p.split > 1 ? launch_hd<96, true>(mq, mql, mk, mv, p, st) : launch_hd<96, false>(mq, mql, mk, mv, p, st);
     }
-    return launch_hd<128>(mq, mql, mk, mv, p, st);
+    return p.split > 1 ? launch_hd<128, true>(mq, mql, mk, mv, p, st) : launch_hd<128, false>(mq, mql, mk, mv, p, st);
 }
 
 }  // namespace forge

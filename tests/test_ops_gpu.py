@@ -483,3 +483,25 @@ def test_rope_forms(L, oracle, hd, heads, rows):
         assert b[skew + x.size:].eq(7.0).all() and b[:skew].eq(7.0).all()
         got.append(v.cpu().numpy().reshape(rows, -1))
     assert np.array_equal(got[0], got[1]) and np.abs(got[0] - ref).max() < 2e-6
+
+
+@pytest.mark.parametrize("hd,nq,nkv", [(64, 9, 3), (96, 4, 4), (128, 6, 2)])
+@pytest.mark.parametrize("m,base,window", [(33, 2000, 0), (200, 1100, 0), (129, 383, 0), (1, 511, 0), (640, 0, 0), (70, 1500, 600), (140, 1500, 65), (300, 900, 1000)])
+def test_attention_batch_split_keys(L, oracle, hd, nq, nkv, m, base, window):
+    """Few query tiles over many keys: two or four CTAs share a tile's keys and put their sums together; rows that see none of a CTA's keys, windows, ragged last tiles."""
+    import torch
+    lib, check = L
+    rng = np.random.default_rng(hd + m + base + window)
+    q = rng.standard_normal((m, nq * hd), dtype=np.float32)
+    k, v = _kv(rng, base + m, nkv, hd, 0.5)
+    kf, vf = k.astype(np.float32), v.astype(np.float32)
+    dq, dk, dv = dev(q), dev(k.view(np.uint16)), dev(v.view(np.uint16))
+    out = torch.full((m, nq * hd), float("nan"), dtype=torch.float32, device="cuda")
+    if window:
+        ref = oracle.attention_sliding_batch(q, oracle.KV_F16, kf, vf, None, None, m, base, window, nq, nkv, hd)
+        check(lib.forge_attention_sliding_batch(out.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), m, base, window, nq, nkv, hd, None))
+    else:
+        ref = oracle.attention_flash_batch(q, oracle.KV_F16, kf, vf, None, None, m, base, nq, nkv, hd)
+        check(lib.forge_attention_flash_batch(out.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), m, base, nq, nkv, hd, None))
+    _sync()
+    assert rel_l2(out.cpu().numpy(), ref) < 2e-5
