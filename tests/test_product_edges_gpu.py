@@ -113,3 +113,27 @@ def test_batched_steps_of_every_size_agree(oracle):
             assert rel_l2(a, b) < 1.2e-4
         kv.close()
     gm.close()
+
+
+@pytest.mark.parametrize("quant,hidden", [(8, 160), (4, 160), (8, 256)])
+def test_small_batched_steps_by_both_products(quant, hidden):
+    """Steps of 2 .. 8 sequences: rows of whole 64-column steps take the tcgen05 products, others the mma.sync one; both agree with single steps to the products' and the
+    fp16 cache's last bits (3e-5 a product, eight of them)."""
+    from forge_llm_b200 import configs, runtime, synth
+    c = configs.tiny(quant, hd=64, nq=4, nkv=2, layers=2, hidden=hidden, ffn=384, vocab=1000)
+    gm = runtime.Model(c, synth.make_weights_bin(c))
+    prompts = [synth.prompt_tokens(c, 5 + 9 * i, seed=70 + i) for i in range(8)]
+    want = []
+    for p in prompts:
+        kv = gm.new_cache(max_seq=100)
+        gm.forward_prefill(p, kv)
+        want.append(gm.forward(int(p[0]), kv))
+        kv.close()
+    for batch in (2, 3, 5, 8):
+        kv = gm.new_cache(max_seq=100, batch=batch)
+        for i in range(batch):
+            gm.forward_prefill(prompts[i], kv, seq=i)
+        got = gm.forward_batch([int(p[0]) for p in prompts[:batch]], kv)
+        assert max(rel_l2(a, b) for a, b in zip(got, want)) < 2.4e-4
+        kv.close()
+    gm.close()
