@@ -211,7 +211,7 @@ TRAFFIC_NOTE = "scaled from one ncu capture of the GEMV kernel (traffic/algorith
 # The prompt's dominant kernel is the gate/up GEMM (tcgen05, SiLU epilogue): one captured launch at m = 1501 read
 # 31.5 MB and wrote 6.2 MB of DRAM (weights 18.9 MB + fp16 hi/lo rows 12.3 MB in; most of its output is still in L2 when
 # it ends); the capture is summarised under profiles/.  Reported for the headline prompt length only.
-PREFILL_GEMM_TRAFFIC = {"c2": (1501, 37.7e6)}
+PREFILL_GEMM_TRAFFIC = {"c2": (1501, 36.8e6)}
 PREFILL_TRAFFIC_NOTE = "dram read + write of one ncu-captured launch of the dominant kernel (gate/up GEMM, m = 1501)"
 
 

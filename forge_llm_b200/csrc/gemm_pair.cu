@@ -20,8 +20,8 @@
 //
 // What bounds it: the tensor pipe (12 products of 96 clocks per K step at 192 tokens = 0.61 us, measured 0.66) and from about 1500 TFLOP/s on the board's power.
 // The one-CTA kernel of gemm_tc5.cu runs a K step as fast but begins and ends every tile with 11-12 us in which the tensor pipe stands still; here they lie
-// under other tiles' products.  us per product, before -> now: Q4_0 2501 tokens 2048 -> 16384 with SiLU 373 -> 320, 8192 -> 2048 206 -> 167, 2048 -> 2048
-// 80 -> 50; 2048 tokens 4096 -> 12288 556 -> 404; Q8_0 1282 tokens 896 -> 9728 with SiLU 88 -> 54, 64 tokens 896 -> 151936 171 -> 71, 896 -> 1152 20.5 -> 12.3.
+// under other tiles' products.  us per product, before -> now: Q4_0 2501 tokens 2048 -> 16384 with SiLU 373 -> 323, 8192 -> 2048 206 -> 168, 2048 -> 2048
+// 80 -> 49; 2048 tokens 4096 -> 12288 556 -> 404; Q8_0 1282 tokens 896 -> 9728 with SiLU 88 -> 53, 64 tokens 896 -> 151936 171 -> 70, 896 -> 1152 20.5 -> 12.3.
 // Tried: threads that store the output themselves (17 us a tile of 192 tokens, longer than its products at K = 896); four epilogue warps (14 us with the SiLU);
 // barriers with cluster-wide ordering (each wait and arrival about 500 clocks: a K step of 1.15 us).
 #include <cuda.h>
